@@ -32,7 +32,9 @@ class Model(C.Structure):
                                           "n_ar_tokens", "reserved")] + \
                [(n, _fp) for n in ("wx", "bx", "wy", "by", "marker", "ar_tokens", "lnf_g", "lnf_b", "wa_t", "ba",
                                    "wb_t", "bb", "mean_bias", "std_bias", "weight_bias", "tc_wa", "tc_wb")] + \
-               [("tc_head_lo", C.c_int32), ("tc_reserved", C.c_int32), ("layers", C.POINTER(LayerWeights))]
+               [("tc_head_lo", C.c_int32), ("tc_reserved", C.c_int32), ("layers", C.POINTER(LayerWeights)),
+                ("seq_w", _fp), ("seq_rank_bytes", C.c_int64), ("seq_vec_off", C.c_int64),
+                ("seq_ranks", C.c_int32), ("seq_reserved", C.c_int32)]
 
 
 class State(C.Structure):
@@ -49,6 +51,9 @@ _i, _p = C.c_int, C.c_void_p
 _SIGNATURES = {
     "artab_prefill": (_i, [C.POINTER(Model), C.POINTER(State), _p, _p, _i, _p]),
     "artab_decode_step": (_i, [C.POINTER(Model), C.POINTER(State), _p, _i, _i, _i, _p, _p, _p, _p, _p, _p]),
+    "artab_sequence_workspace": (C.c_int64, [C.POINTER(Model), C.POINTER(State)]),
+    "artab_decode_sequence": (_i, [C.POINTER(Model), C.POINTER(State), _p, C.c_int64, _i, _i, _i, _i, _p, _p, _p, _p, _p,
+                                   _p, C.c_int64, _p]),
     "artab_decode_embedded": (_i, [C.POINTER(Model), C.POINTER(State), _p, _i, _i, _p, _p]),
     "artab_teacher_forcing": (_i, [C.POINTER(Model), C.POINTER(State), _p, _p, _i, _i, _p, _p]),
     "artab_forward_masked": (_i, [C.POINTER(Model), C.POINTER(State), _p, _p, _p, _p, _i, _i, _i, _p, _p, _p]),

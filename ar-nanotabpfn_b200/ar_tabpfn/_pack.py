@@ -140,6 +140,7 @@ class PackedModel:
         m.layers = C.cast(self._layers, C.POINTER(_lib.LayerWeights))
         self.struct = m
         self._pack_tensor_core(embedder, backbone, head, target)
+        self._pack_sequence(dict(items), target)
 
     def _pack_tensor_core(self, embedder, backbone, head, target):
         """bf16 hi/lo tiles for the tcgen05 per-token chain (d_model in {64,128,192}, d_ff % 128 == 0,
@@ -197,6 +198,52 @@ class PackedModel:
         self.struct.tc_wa = base + 2 * offs["tc_wa"]
         self.struct.tc_wb = base + 2 * offs["tc_wb"]
         self.struct.tc_head_lo = head_bits
+
+    def _pack_sequence(self, w, target):
+        """Weight streams of the whole-sequence decode: per cluster rank the slices of every matrix in the
+        order of use (layer by layer: fold, Q|K|V of the rank's heads | out-projection, MLP; then the head).
+        A slice [K][N] is a sequence of units of 32 k x 16 columns, k blocks outermost; inside a unit element
+        (k = 4s + e, n = 4g + c) sits at [c][s][g][e].  ``w`` holds the matrices as [in][out]."""
+        D, Dff, H, Dh, K = self.d_model, self.d_ff, self.n_heads, self.head_dim, self.n_comp
+        ranks = max(c for c in range(1, 9) if H % c == 0)
+        self.seq_flat = None
+        if D % 64 or Dff % ranks or D // ranks % 16 or Dff // ranks % 32:
+            return
+        ds, hs, qs = D // ranks, Dff // ranks, H // ranks * Dh
+        wb = torch.zeros(Dff, (3 * K + 15) // 16 * 16, dtype=torch.float64)
+        wb[:, :3 * K] = w["wb_t"]
+        unit = lambda m: (m.reshape(m.shape[0] // 32, 8, 4, m.shape[1] // 16, 4, 4).permute(0, 3, 5, 1, 4, 2)
+                          .to(torch.float32).reshape(-1))
+        streams = []
+        for r in range(ranks):
+            cols = lambda m, n: m[:, r * n:(r + 1) * n]
+            parts = []
+
+            def pre(i):
+                parts.append(cols(w[f"{i}.wf_t"], ds))
+                parts.append(torch.cat([cols(m, qs) for m in w[f"{i}.wqkv_t"].split(D, dim=1)], dim=1))
+
+            pre(0)
+            for i in range(self.n_layers):
+                parts += [cols(w[f"{i}.wo_t"], ds), cols(w[f"{i}.w1_t"], hs), w[f"{i}.w2_t"][r * hs:(r + 1) * hs]]
+                if i + 1 < self.n_layers:
+                    pre(i + 1)
+            parts += [cols(w["wa_t"], hs), wb[r * hs:(r + 1) * hs]]
+            # after the matrices: per layer LayerNorm 1 / 2 vectors, b2, LayerNorm 3 vectors, b1 slice; final
+            # LayerNorm, first bias of the head (slice)
+            part = lambda v: v[r * hs:(r + 1) * hs]
+            vec = []
+            for i in range(self.n_layers):
+                vec += [w[f"{i}.{k}"] for k in ("ln1_g", "ln1_b", "ln2_g", "ln2_b", "b2", "ln3_g", "ln3_b")] + [part(w[f"{i}.b1"])]
+            vec += [w["lnf_g"], w["lnf_b"], part(w["ba"])]
+            mats = [unit(p) for p in parts]
+            self.struct.seq_vec_off = 4 * sum(m.numel() for m in mats)
+            streams.append(torch.cat(mats + [v.reshape(-1).to(torch.float32) for v in vec]))
+        flat = torch.stack(streams)
+        self.struct.seq_ranks = ranks
+        self.struct.seq_rank_bytes = 4 * flat.shape[1]
+        self.seq_flat = flat.to(target)
+        self.struct.seq_w = self.seq_flat.data_ptr()
 
     @property
     def ref(self):

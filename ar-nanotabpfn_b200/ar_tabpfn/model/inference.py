@@ -385,20 +385,40 @@ class ARTabPFNPredictor:
         K = int(self.head.num_components)
         if expo.shape != (Nt, B, K) or normal.shape != (Nt, B):
             raise ValueError("variates must be (expo [Nt,B,K], normal [Nt,B])")
-        xt = self._dev32(x_target, device)
-        samples = torch.zeros(B, Nt, device=device, dtype=torch.float32)
-        logdens = torch.zeros(B, Nt, device=device, dtype=torch.float32)
-        comp = torch.zeros(B, Nt, device=device, dtype=torch.int32)
+        samples = torch.empty(B, Nt, device=device, dtype=torch.float32)
+        logdens = torch.empty(B, Nt, device=device, dtype=torch.float32)
+        comp = torch.empty(B, Nt, device=device, dtype=torch.int32)
         pm = self._packed(device)
         st = self._state
         stream = _lib.stream_ptr()
-        for t in range(Nt):
+
+        def variates_ready(t):
+            """Decode step t waits for its chunk of draws; the host stays one chunk ahead of the steps."""
             if drawn is not None and t % 16 == 0:
-                issue_draws(t + 16)      # the host stays one chunk ahead of the decode steps it launches
+                issue_draws(t + 16)
                 torch.cuda.current_stream(device).wait_event(drawn[t])
-            _lib.check(lib.artab_decode_step(pm.ref, C.byref(st), _lib.ptr(xt), F, Nt, t, _lib.ptr(samples),
-                                             _lib.ptr(expo[t]), _lib.ptr(normal[t]), _lib.ptr(logdens),
-                                             _lib.ptr(comp), stream))
+
+        need = int(lib.artab_sequence_workspace(pm.ref, C.byref(st)))
+        if need > 0:
+            # one launch per chunk of draws (one in all when they are given)
+            if x_target.is_cuda and B > 1 and x_target.stride(0) == 0:
+                xt, xt_stride = self._dev32(x_target[:1], device), 0   # the same rows for every stream
+            else:
+                xt, xt_stride = self._dev32(x_target, device), Nt * F
+            ws = self._alloc("seq_ws", (need,), torch.uint8)
+            for t in range(0, Nt, 16 if drawn is not None else Nt):
+                variates_ready(t)
+                t1 = min(t + 16, Nt) if drawn is not None else Nt
+                _lib.check(lib.artab_decode_sequence(pm.ref, C.byref(st), _lib.ptr(xt), xt_stride, F, Nt, t, t1,
+                                                     _lib.ptr(samples), _lib.ptr(expo), _lib.ptr(normal),
+                                                     _lib.ptr(logdens), _lib.ptr(comp), _lib.ptr(ws), need, stream))
+        else:
+            xt = self._dev32(x_target, device)
+            for t in range(Nt):
+                variates_ready(t)
+                _lib.check(lib.artab_decode_step(pm.ref, C.byref(st), _lib.ptr(xt), F, Nt, t, _lib.ptr(samples),
+                                                 _lib.ptr(expo[t]), _lib.ptr(normal[t]), _lib.ptr(logdens),
+                                                 _lib.ptr(comp), stream))
         self.buffer_len = int(st.buffer_len)
         self.seq_len = self.context_len + self.buffer_len
         self.last_logdens = logdens

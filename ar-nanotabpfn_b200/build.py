@@ -15,7 +15,12 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libartab_b200.so")
-SOURCES = ["api.cu", "dense_simt.cu", "attn_simt.cu", "attn_tc.cu", "buf_mma.cu", "noalloc.cu", "dense_tc.cu"]
+# (source, object name, extra defines)
+SOURCES = [(f, f[:-3], []) for f in ("api.cu", "dense_simt.cu", "attn_simt.cu", "attn_tc.cu", "buf_mma.cu", "noalloc.cu",
+                                     "dense_tc.cu", "seq.cu")]
+# the whole-sequence kernel has many variants: one compiler process per cache type and head size
+SOURCES += [("seq_simt.cu", f"seq_simt_{'bf16' if b else 'f32'}_{dh}", [f"-DARTAB_SEQ_BF16={b}", f"-DARTAB_SEQ_DH={dh}"])
+            for b in (0, 1) for dh in (16, 32, 64)]
 FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
@@ -38,9 +43,15 @@ def build(force: bool = False, verbose: bool = False) -> str:
     objs = []
     procs = []
     os.makedirs(os.path.join(HERE, "build"), exist_ok=True)
-    for src in SOURCES:
-        obj = os.path.join(HERE, "build", src.replace(".cu", ".o"))
-        cmd = [nvcc, *FLAGS, "-c", os.path.join(CSRC, src), "-o", obj]
+    headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".cuh")]
+    newest = max(map(os.path.getmtime, [*headers, os.path.join(ROOT, "include", "artab.h"), __file__]))
+    for src, name, defines in SOURCES:
+        obj = os.path.join(HERE, "build", name + ".o")
+        if not force and os.path.exists(obj) and os.path.getmtime(obj) > max(
+                newest, os.path.getmtime(os.path.join(CSRC, src))):
+            objs.append(obj)
+            continue
+        cmd = [nvcc, *FLAGS, *defines, "-c", os.path.join(CSRC, src), "-o", obj]
         if verbose:
             cmd.insert(1, "-Xptxas=-v")
         procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))

@@ -10,6 +10,7 @@
 
 #include "attn.cuh"
 #include "dense.cuh"
+#include "seq.cuh"
 
 namespace artab {
 
@@ -87,6 +88,25 @@ int check_launch(const char* what) {
   return ARTAB_OK;
 }
 
+// The tensor-core chain reads attn / x1 in the lane-major layout (workspaces padded to 128 rows).
+bool chain_on_tc(const artab_model* m, const artab_state* st) {
+  if (st->dtype != ARTAB_BF16 || !m->tc_wa || !m->tc_wb) return false;
+  for (int l = 0; l < m->n_layers; ++l)
+    if (!m->layers[l].tc_wo || !m->layers[l].tc_w1 || !m->layers[l].tc_w2 || !m->layers[l].tc_wf ||
+        !m->layers[l].tc_wqkv)
+      return false;
+  DenseArgs probe;
+  memset(&probe, 0, sizeof(probe));
+  probe.D = m->d_model;
+  probe.Dff = m->d_ff;
+  probe.n_comp = m->n_comp;
+  probe.kv.dtype = st->dtype;
+  probe.do_head = 1;
+  probe.tc_wa = m->tc_wa;
+  probe.tc_wb = m->tc_wb;
+  return dense_tc_applicable(probe);
+}
+
 namespace {
 
 constexpr int kSMs = 148;
@@ -160,25 +180,6 @@ int plan_splits(int dtype, int head_dim, int rows, int rows_per_group, int n_gro
     }
   }
   return best;
-}
-
-// The tensor-core chain reads attn / x1 in the lane-major layout (workspaces padded to 128 rows).
-bool chain_on_tc(const artab_model* m, const artab_state* st) {
-  if (st->dtype != ARTAB_BF16 || !m->tc_wa || !m->tc_wb) return false;
-  for (int l = 0; l < m->n_layers; ++l)
-    if (!m->layers[l].tc_wo || !m->layers[l].tc_w1 || !m->layers[l].tc_w2 || !m->layers[l].tc_wf ||
-        !m->layers[l].tc_wqkv)
-      return false;
-  DenseArgs probe;
-  memset(&probe, 0, sizeof(probe));
-  probe.D = m->d_model;
-  probe.Dff = m->d_ff;
-  probe.n_comp = m->n_comp;
-  probe.kv.dtype = st->dtype;
-  probe.do_head = 1;
-  probe.tc_wa = m->tc_wa;
-  probe.tc_wb = m->tc_wb;
-  return dense_tc_applicable(probe);
 }
 
 int run_ctx(const artab_model* m, const artab_state* st, int layer, int rows, int rows_per_group, int n_splits,
@@ -552,6 +553,45 @@ int artab_decode_step(const artab_model* m, artab_state* st, const float* xt, in
   rc = decode_common(m, st, n_new, last, chain_on_tc(m, st), s);
   if (rc) return rc;
   st->buffer_len += n_new - 1;
+  return ARTAB_OK;
+}
+
+int64_t artab_sequence_workspace(const artab_model* m, const artab_state* st) {
+  if (check_model(m) || check_state(m, st)) return 0;
+  return seq_applicable(m, st) ? (int64_t)seq_workspace_bytes(m, st) : 0;
+}
+
+int artab_decode_sequence(const artab_model* m, artab_state* st, const float* xt, int64_t xt_stride, int n_feat,
+                          int n_targets, int t0, int t1, float* samples, const float* expo, const float* normal,
+                          float* logdens, int32_t* comp, void* workspace, int64_t workspace_bytes, void* stream) {
+  int rc = check_model(m);
+  if (rc) return rc;
+  rc = check_state(m, st);
+  if (rc) return rc;
+  ARTAB_REQUIRE(xt && samples && expo && normal && workspace && n_feat > 0 && xt_stride >= 0, ARTAB_EINVAL,
+                "decode_sequence: bad argument");
+  ARTAB_REQUIRE(t0 >= 0 && t1 > t0 && t1 <= n_targets, ARTAB_EINVAL, "decode_sequence: bad target range");
+  ARTAB_REQUIRE(t1 == 1 || (t1 - 1 <= st->max_buf && st->kv_buf), ARTAB_ECAPACITY,
+                "Shared-context buffer cache exceeded; increase max buffer length.");
+  ARTAB_REQUIRE(st->buffer_len == (t0 ? t0 - 1 : 0), ARTAB_EINVAL, "decode_sequence: target %d does not follow %d buffer rows",
+                t0, st->buffer_len);
+  SeqCall c;
+  c.xt = xt;
+  c.xt_stride = (size_t)xt_stride;
+  c.n_feat = n_feat;
+  c.n_targets = n_targets;
+  c.t0 = t0;
+  c.t1 = t1;
+  c.samples = samples;
+  c.expo = expo;
+  c.normal = normal;
+  c.logdens = logdens;
+  c.comp = comp;
+  c.workspace = workspace;
+  c.workspace_bytes = (size_t)workspace_bytes;
+  rc = launch_seq(m, st, c, (cudaStream_t)stream);
+  if (rc) return rc;
+  st->buffer_len = t1 - 1;
   return ARTAB_OK;
 }
 

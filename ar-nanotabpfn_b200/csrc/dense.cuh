@@ -64,5 +64,6 @@ int launch_embed(const EmbedArgs& a, cudaStream_t s);
 int launch_dense(const DenseArgs& a, cudaStream_t s);     // picks the tensor-core chain when it applies
 int launch_dense_tc(const DenseArgs& a, cudaStream_t s);  // tcgen05 chain (bf16 mode)
 bool dense_tc_applicable(const DenseArgs& a);
+bool chain_on_tc(const artab_model* m, const artab_state* st);  // every dense launch of this model takes the tcgen05 chain
 
 }  // namespace artab

@@ -7,8 +7,8 @@
  *     throws, never synchronises the device and never allocates device memory.
  *     Buffers and workspaces are passed in by the caller, with one exception:
  *     artab_context_attention_noalloc keeps its partials in an array inside the library.
- *   - The whole-path entry points (artab_prefill, artab_decode_step, artab_decode_embedded,
- *     artab_teacher_forcing, artab_forward_masked) overlap their own kernels with programmatic
+ *   - The whole-path entry points (artab_prefill, artab_decode_step, artab_decode_sequence,
+ *     artab_decode_embedded, artab_teacher_forcing, artab_forward_masked) overlap their own kernels with programmatic
  *     dependent launch; the single-operator entry points launch plainly, because they cannot know
  *     what the caller enqueued before them.
  *   - All data pointers are device pointers unless a comment says "host".
@@ -113,6 +113,13 @@ typedef struct artab_model {
   int32_t tc_head_lo;        /* bit 0 wa, bit 1 wb */
   int32_t tc_reserved;
   const artab_layer_weights* layers; /* HOST pointer to n_layers entries */
+  /* whole-sequence decode (NULL: artab_decode_sequence is not available): per cluster rank one contiguous
+   * stream of the matrix slices that rank uses, in the order of use, fp32 in units of 32 k x 16 columns (_pack.py);
+   * seq_ranks is the largest divisor of n_heads that is at most 8 */
+  const void* seq_w;
+  int64_t seq_rank_bytes, seq_vec_off;  /* bytes per rank; where its LayerNorm and bias vectors start */
+  int32_t seq_ranks;
+  int32_t seq_reserved;
 } artab_model;
 
 /* ------------------------------------------------------------------------- */
@@ -187,6 +194,21 @@ ARTAB_API int artab_decode_step(const artab_model* m, artab_state* st, const flo
  * Replaces ARTabPFNPredictor.transformer_decode (ar_tabpfn/model/inference.py:226-276). */
 ARTAB_API int artab_decode_embedded(const artab_model* m, artab_state* st, const float* x_in, int n_new, int commit,
                           float* z_out, void* stream);
+
+/* Bytes of workspace artab_decode_sequence needs for this model and state, 0 where it does not apply (the
+ * caller then loops over artab_decode_step). */
+ARTAB_API int64_t artab_sequence_workspace(const artab_model* m, const artab_state* st);
+
+/* Targets [t0, t1) of the sampling loop in ONE launch, every stream walked through all its targets on chip:
+ * the same results as artab_decode_step called for t0 .. t1-1, up to fp32 summation order.
+ *   xt: features of stream b at xt + b * xt_stride, [Nt][F] (xt_stride 0: the same rows for every stream);
+ *   expo [Nt][B][K], normal [Nt][B]: random numbers of ALL targets; the rest as in artab_decode_step.
+ * A sequence may be decoded in several consecutive parts; the call with t0 = 0 lays the context out in
+ * `workspace`, which must stay untouched until the last part.
+ * Replaces the loop of ARTabPFNPredictor.sample_sequence (ar_tabpfn/model/inference.py:323-366). */
+ARTAB_API int artab_decode_sequence(const artab_model* m, artab_state* st, const float* xt, int64_t xt_stride, int n_feat,
+                          int n_targets, int t0, int t1, float* samples, const float* expo, const float* normal,
+                          float* logdens, int32_t* comp, void* workspace, int64_t workspace_bytes, void* stream);
 
 /* Teacher-forced joint log density of all targets in one pass:
  * tokens [Buffer_0..Buffer_{Nt-1}, Target_0..Target_{Nt-1}] per stream, block-causal

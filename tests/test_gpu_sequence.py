@@ -1,0 +1,72 @@
+"""The one-launch decode of a whole sampling job against the CPU oracle: every kernel variant (streams per
+cluster, head size, cache type, shared or own contexts) at the sizes where its tiles end: context tiles of
+32 keys, private keys of 32 in four parts, clusters with a stream missing, several heads per CTA."""
+import pytest
+import torch
+
+import artab_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+# d_model, heads, layers, d_ff, components, streams, context rows, targets, shared
+CASES = [
+    (64, 4, 2, 128, 5, 1, 1, 3, True),          # one key, one stream
+    (64, 4, 1, 128, 20, 5, 33, 6, True),        # head size 16, twenty components
+    (64, 2, 1, 128, 5, 37, 31, 4, True),        # two CTAs per cluster, context one key short of a tile
+    (64, 1, 1, 64, 5, 3, 64, 5, True),          # one head: no cluster to form, the launch-per-layer path
+    (128, 4, 2, 256, 5, 130, 40, 4, True),      # four streams per cluster, the last cluster not full
+    (128, 2, 1, 256, 3, 9, 70, 5, False),       # head size 64, own contexts
+    (128, 8, 1, 512, 5, 200, 30, 3, True),      # eight CTAs, many streams: the widest variant
+    (192, 6, 1, 768, 5, 20, 65, 4, False),      # own contexts, head size 32
+    (192, 12, 1, 192, 5, 3, 20, 3, True),       # two heads of 16 per CTA
+    (64, 4, 1, 128, 5, 6, 50, 140, True),       # private keys beyond one round of the four parts
+    (64, 4, 1, 128, 5, 420, 20, 3, False),      # more streams than one wave of clusters holds
+]
+
+
+@pytest.mark.parametrize("precision", ["fp32", "bf16"])
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "d%d_h%d_l%d_ff%d_k%d_b%d_nc%d_nt%d_%s" % (*c[:8], "shared" if c[8] else "own"))
+def test_sequence_matches_oracle(case, precision):
+    import ar_tabpfn
+    D, H, L, Dff, K, B, Nc, Nt, shared = case
+    torch.manual_seed(3 + D + Nc)
+    m = ar_tabpfn.ARTabPFN(d_model=D, n_heads=H, n_layers=L, d_ff=Dff, num_features=5, num_components=K).eval()
+    r = lambda t: t.to(torch.bfloat16).float()
+    with torch.no_grad():
+        for p in m.parameters():
+            p.copy_(r(p))
+            p.requires_grad_(False)
+    sd = {k: v.clone() for k, v in m.state_dict().items()}
+    n = 1 if shared else B
+    xs, ys = zip(*[orc.make_dataset(7 * b + 1, Nc + Nt, 5) for b in range(n)])
+    x, y = r(torch.stack(xs)).expand(B, -1, -1), r(torch.stack(ys)).expand(B, -1)
+    xc, yc, xt = x[:, :Nc], y[:, :Nc], x[:, Nc:]
+    # the component of every draw is fixed by a wide margin, so that rounding cannot pick another one
+    g = torch.Generator().manual_seed(5)
+    expo = torch.rand(Nt, B, K, generator=g) + 0.5
+    expo.scatter_(2, torch.randint(K, (Nt, B, 1), generator=g), 1e-5)
+    normal = torch.randn(Nt, B, generator=g)
+    run = lambda o, f: o.sample_sequence(*(f(t) for t in (xc, yc, xt, expo, normal)), shared=shared)
+    want_y, want_ld, want_c = run(orc.OraclePredictor(sd, H), lambda t: t)
+    pred = ar_tabpfn.ARTabPFNPredictor.from_trained_model(
+        m.cuda(), backend="triton_shared_context" if shared else "flex_attention", precision=precision)
+    c = lambda t: t.cuda()
+    got_y = pred.sample_sequence(c(xc), c(yc), c(xt), variates=(c(expo), c(normal))).cpu()
+    got_ld = pred.last_logdens.cpu()
+    assert pred.last_status() == 0
+    assert torch.equal(pred.last_components.cpu(), want_c)
+    # Bounds: the bar of the mode plus four times what the mode's arithmetic moves the oracle itself by on
+    # this stream (root mean square over its targets): fp32 against fp64; bf16 storage of q / k / v and bf16
+    # softmax numerators emulated in the oracle, three realisations.
+    if precision == "fp32":
+        d = lambda t: t.double()
+        alt = [run(orc.OraclePredictor({k: d(v) for k, v in sd.items()}, H), d)]
+        bar_y, bar_ld = 1e-5, 3e-5
+    else:
+        alt = [run(orc.OraclePredictor(sd, H, orc.Emulation(qkv=True, p=True, jitter=j)), lambda t: t) for j in (0, 1, 2)]
+        bar_y, bar_ld = 2e-3, 2e-3
+    for got, want, k, bar in ((got_y, want_y, 0, bar_y), (got_ld, want_ld, 1, bar_ld)):
+        noise = torch.stack([(a[k].double() - want.double()).pow(2).mean(1, keepdim=True) for a in alt]).mean(0).sqrt()
+        err = (got.double() - want.double()).abs()
+        bound = bar * (1 + want.double().abs()) + 4 * noise
+        assert bool((err <= bound).all()), (k, float(err.max()), float((err / bound).max()))
