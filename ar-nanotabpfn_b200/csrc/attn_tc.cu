@@ -51,14 +51,15 @@ struct WaitCtl {
 struct __align__(1024) Smem {
   uint8_t q[BM * 64];               // [128 rows][32 bf16], 64-byte swizzle
   uint8_t k[NSTAGE][BN * 64];       // [128 keys][32 bf16], 64-byte swizzle
-  uint8_t v[NSTAGE][2][64 * 128];   // V^T hi|lo: two boxes of [64 rows][64 keys], 128-byte swizzle
+  uint8_t v[NSTAGE][2][64 * 128];   // V^T hi|lo: two boxes of [64 rows][64 keys], 128-byte swizzle; NATURAL: [128 keys][32]
   uint64_t q_full, s_full, p_full, o_full;
   uint64_t s_free;                  // every softmax thread has read its scores of the current tile
+  uint64_t verdict;                 // the one-pass walk is over and `redo` says whether it has to be repeated
   uint64_t kv_full[NSTAGE], kv_empty[NSTAGE];
   float xmax[2][2][BM];             // row maxima exchanged between the two softmax warpgroups
   float xsum[BM];                   // row sum of the second warpgroup (epilogue)
   uint32_t tmem_base;
-  uint32_t pad_;
+  int redo;
   WaitCtl ctl;
 };
 
@@ -106,6 +107,13 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* tm, in
       : "memory");
 }
 
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* tm, int c0, int c1, int c2, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(smem_u32(dst)), "l"(tm), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
+
 // K-major shared-memory matrix descriptor: rows of `swizzle` bytes, 8-row groups `sbo` bytes apart.
 constexpr uint64_t kLayoutSw128 = 2, kLayoutSw64 = 4;
 __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t sbo_bytes, uint64_t layout) {
@@ -118,8 +126,9 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t sbo_bytes
 }
 
 // kind::f16 instruction descriptor: fp32 accumulate, bf16 A and B, both K-major.
-constexpr uint32_t make_idesc(int M, int N) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+// b_mn: B is stored with N contiguous (V rows as they are: [key][dim]) instead of K contiguous.
+constexpr uint32_t make_idesc(int M, int N, bool b_mn = false) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | (b_mn ? 1u << 16 : 0u) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
 __device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
@@ -177,7 +186,7 @@ __device__ __forceinline__ float ex2_approx(float x) {
 // 7.5e-5, far below the bf16 rounding of P), and n added into the exponent field.  x is clamped at
 // -125 (the result is then ~2e-38, i.e. nothing); x stays below ~2^4 here (lazy maximum).
 #ifndef ARTAB_POLY_EXP_OF_8
-#define ARTAB_POLY_EXP_OF_8 2   // of every 8 score pairs this many take the FMA-pipe exponential (measured best: 0 -> 88.2 us, 2 -> 82.2, 3 -> 85.3, 4 -> 89.7 at 4096 rows x 8192 keys)
+#define ARTAB_POLY_EXP_OF_8 2   // of every 8 score pairs this many take the FMA-pipe exponential (measured best in both forms of the tile; one-pass, 8192 rows x 16384 keys: 2 -> 242 us, 1 -> 250, 3 -> 255, 0 -> 266)
 #endif
 __device__ __forceinline__ float2 ex2_poly2(float2 x) {
   x.x = fmaxf(x.x, -125.0f);
@@ -249,7 +258,7 @@ constexpr float kLazyMax = 8.0f;
 // warpgroup its half of the 64 output columns: one tcgen05.ld / st round trip), which on ordinary
 // data happens on the first tiles only.  The result does not depend on when m is raised: the final
 // O / l and lse = m + log2(l) are exact in m.
-template <bool MASKED>
+template <bool MASKED, bool NATURAL>
 __device__ __forceinline__ bool softmax_tile(Smem* sm, uint32_t t_row, int wg, int row, int parity, float sc,
                                              int n_valid, float& m, float& l, bool first,
                                              volatile int* abort_flag) {
@@ -309,7 +318,7 @@ __device__ __forceinline__ bool softmax_tile(Smem* sm, uint32_t t_row, int wg, i
     if (c == 0 && !first) {
       ok = mbar_wait(&sm->o_full, parity ^ 1, abort_flag);
       tc_fence_after();
-      if (__any_sync(0xffffffffu, raise)) {  // rare: rescale this warpgroup's half of the accumulated O
+      if (!(NATURAL && wg == 1) && __any_sync(0xffffffffu, raise)) {  // rare: rescale this warpgroup's half of the accumulated O
         uint32_t o[32];
         tmem_ld32(t_row + kColO + 32 * wg, o);
         tmem_wait_ld();
@@ -324,6 +333,81 @@ __device__ __forceinline__ bool softmax_tile(Smem* sm, uint32_t t_row, int wg, i
   return ok;
 }
 
+// The same tile in ONE pass: exponentials against the reference the first tile left, whatever this tile's
+// maximum is.  No maximum pass, no exchange between the warpgroups, no rescale: the scores are read once.
+// That is exact in the reference (O / l and m + log2(l) do not depend on it) as long as nothing overflows:
+// the numerators may grow to kOnePassMax, and a row that passes that shows in its sum, upon which the CTA
+// walks its keys again with the two-pass form.  Two passes per tile -> one, 6 heads: 4096 rows x 8192 keys
+// 79.5 -> 69.5 us, 8192 x 16384 285 -> 242 us (2.83 -> 3.33e12 exponentials per second), 64 contexts of 2048
+// rows attending to themselves 595 -> 515 us.  Measured beside it and dropped: P and P . V in two chunks with
+// barriers of their own (261 us at 8192 x 16384), fewer reads of the clock in the waits (no change).
+constexpr float kOnePassMax = 1.2676506e30f;  // 2^100
+__device__ __forceinline__ float2 pk_fma(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\t"
+      "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
+      "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 pk_add(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rd;\n\t"
+      "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
+      "add.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+template <bool MASKED>
+__device__ __forceinline__ bool softmax_tile_one_pass(Smem* sm, uint32_t t_row, int wg, uint32_t o_parity, float sc, int n_valid,
+                                                      float m, float& l, volatile int* abort_flag) {
+  const int col0 = 64 * wg;
+  const float2 sc2 = make_float2(sc, sc), nm2 = make_float2(-m, -m);
+  float2 sum = make_float2(0.f, 0.f);
+  bool ok = true;
+#pragma unroll 1
+  for (int c = 0; c < 2; ++c) {
+    uint32_t r[32], pk[16];
+    tmem_ld32(t_row + kColS + col0 + 32 * c, r);
+    tmem_wait_ld();
+    if (c == 1) {  // the scores are in registers: the next tile's Q.K^T may overwrite them
+      tc_fence_before();
+      mbar_arrive(&sm->s_free);
+    }
+#pragma unroll
+    for (int i = 0; i < 32; i += 2) {
+      float2 x = pk_fma(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), sc2, nm2);
+      float2 e;
+      if (((i >> 1) & 7) < ARTAB_POLY_EXP_OF_8) {
+        x.x = fminf(x.x, 126.0f);   // beyond that the exponent field would wrap; the sum tells of it all the same
+        x.y = fminf(x.y, 126.0f);
+        e = ex2_poly2(x);
+      } else {
+        e.x = ex2_approx(x.x);
+        e.y = ex2_approx(x.y);
+      }
+      if (MASKED) {
+        if (col0 + 32 * c + i >= n_valid) e.x = 0.f;
+        if (col0 + 32 * c + i + 1 >= n_valid) e.y = 0.f;
+      }
+      sum = pk_add(sum, e);
+      pk[i >> 1] = pack_bf16(e.x, e.y);
+    }
+    if (c == 0) {  // P has one buffer: the previous tile's P . V must have read it
+      ok = mbar_wait(&sm->o_full, o_parity, abort_flag);
+      tc_fence_after();
+    }
+    tmem_st16(t_row + kColP + 32 * wg + 16 * c, pk);
+  }
+  l += sum.x + sum.y;
+  return ok;
+}
+
+// NATURAL: K and V as a caller of the functional operators holds them, [heads][keys][32] bf16 with exact V: no
+// packing pass in front, P . V has 32 columns.
+template <bool NATURAL>
 __global__ void __launch_bounds__(kThreads, 2)
 ctx_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const TcParams p) {
@@ -369,6 +453,8 @@ ctx_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     mbar_init(&sm->p_full, 256);
     mbar_init(&sm->o_full, 1);
     mbar_init(&sm->s_free, 256);
+    mbar_init(&sm->verdict, 256);
+    sm->redo = 0;
     for (int s = 0; s < NSTAGE; ++s) {
       mbar_init(&sm->kv_full[s], 1);
       mbar_init(&sm->kv_empty[s], 1);
@@ -399,26 +485,36 @@ ctx_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     if (lane == 0) {
       const int krow0 = (g * p.n_heads + h) * p.n_ctx_pad;
       const int vrow0 = (g * p.n_heads + h) * 2 * DH;
-      auto load_kv = [&](int j) {
-        const int st = j % NSTAGE;
+      int issued = 0;
+      auto load_kv = [&](int st, int j) {
         const int key0 = (tile_begin + j) * BN;
+        if constexpr (NATURAL) {  // rows past a head's last key read as zero
+          mbar_expect_tx(&sm->kv_full[st], 2 * BN * 64);
+          tma_load_3d(sm->k[st], &tm_k, 0, key0, h, &sm->kv_full[st]);
+          tma_load_3d(sm->v[st][0], &tm_v, 0, key0, h, &sm->kv_full[st]);
+          return;
+        }
         mbar_expect_tx(&sm->kv_full[st], BN * 64 + 2 * 64 * 128);
         tma_load_2d(sm->k[st], &tm_k, 0, krow0 + key0, &sm->kv_full[st]);
         tma_load_2d(sm->v[st][0], &tm_v, key0, vrow0, &sm->kv_full[st]);
         tma_load_2d(sm->v[st][1], &tm_v, key0 + 64, vrow0, &sm->kv_full[st]);
       };
+      // load number i of the CTA (the second walk over the keys, if any, continues the count)
+      auto put = [&](int i) { load_kv(i % NSTAGE, i < nt ? i : i - nt); };
       // the first ring of K/V tiles may be fetched while the preceding kernel (which produces Q) runs
-      int issued = 0;
       const int early = p.kv_stable ? min(nt, NSTAGE) : 0;
-      for (; issued < early; ++issued) load_kv(issued);
+      for (; issued < early; ++issued) put(issued);
       dep_wait();
       mbar_expect_tx(&sm->q_full, BM * 64);
       tma_load_2d(sm->q, &tm_q, h * DH, (int)(group_row0 + m0), &sm->q_full);
-      for (int j = issued; j < nt; ++j) {
-        if (j >= NSTAGE && !mbar_wait(&sm->kv_empty[j % NSTAGE], ((j / NSTAGE) + 1) & 1, abort_flag)) break;
-        load_kv(j);
-        issued = j + 1;
-      }
+      auto walk = [&](int end) {
+        for (; issued < end; ++issued) {
+          if (issued >= NSTAGE && !mbar_wait(&sm->kv_empty[issued % NSTAGE], ((issued / NSTAGE) + 1) & 1, abort_flag)) return;
+          put(issued);
+        }
+      };
+      walk(nt);
+      if (nt > 1 && mbar_wait(&sm->verdict, 0, abort_flag) && *(volatile int*)&sm->redo) walk(2 * nt);
       if (*abort_flag) {  // drain our own copies before the CTA may exit
         {
           const long long t0 = clock64();
@@ -436,13 +532,13 @@ ctx_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     // ------------------------------- MMA issuer -------------------------------
     if (lane == 0) {
       constexpr uint32_t idesc_qk = make_idesc(BM, BN);
-      constexpr uint32_t idesc_pv = make_idesc(BM, 2 * DH);
+      constexpr uint32_t idesc_pv = NATURAL ? make_idesc(BM, DH, true) : make_idesc(BM, 2 * DH);
       bool ok = mbar_wait(&sm->q_full, 0, abort_flag);
       const uint32_t q_addr = smem_u32(sm->q);
       // S = Q . K^T of tile j   (M 128, N 128, K 32 = two k-steps of 16 bf16 = 32 bytes)
-      auto issue_qk = [&](int j) -> bool {
-        const int st = j % NSTAGE;
-        if (!mbar_wait(&sm->kv_full[st], (j / NSTAGE) & 1, abort_flag)) return false;
+      auto issue_qk = [&](int i) -> bool {  // i counts the tiles of both walks
+        const int st = i % NSTAGE;
+        if (!mbar_wait(&sm->kv_full[st], (i / NSTAGE) & 1, abort_flag)) return false;
         tc_fence_after();
         const uint32_t k_addr = smem_u32(sm->k[st]);
 #pragma unroll
@@ -452,29 +548,44 @@ ctx_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         if (!p.drop_score_commits) umma_commit(&sm->s_full);
         return true;
       };
-      ok = ok && issue_qk(0);
-      for (int j = 0; ok && j < nt; ++j) {
-        const int st = j % NSTAGE;
-        // The next tile's scores are computed while the softmax threads still turn this tile's
-        // into P: they release S as soon as their last score is in registers.
-        if (j + 1 < nt) {
-          ok = mbar_wait(&sm->s_free, j & 1, abort_flag);
+      for (int walk = 0; ok && walk < 2; ++walk) {
+        const int i0 = walk * nt;
+        if (walk == 1 && (nt == 1 || !mbar_wait(&sm->verdict, 0, abort_flag) || !*(volatile int*)&sm->redo ||
+                          !mbar_wait(&sm->s_free, (i0 - 1) & 1, abort_flag)))
+          break;
+        tc_fence_after();
+        ok = issue_qk(i0);
+        for (int i = i0; ok && i < i0 + nt; ++i) {
+          const int st = i % NSTAGE;
+          // The next tile's scores are computed while the softmax threads still turn this tile's
+          // into P: they release S as soon as their last score is in registers.
+          if (i + 1 < i0 + nt) {
+            ok = mbar_wait(&sm->s_free, i & 1, abort_flag);
+            if (!ok) break;
+            tc_fence_after();
+            ok = issue_qk(i + 1);
+            if (!ok) break;
+          }
+          // softmax writes P -> O (+)= P . [V_hi | V_lo]
+          ok = mbar_wait(&sm->p_full, i & 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
-          ok = issue_qk(j + 1);
-          if (!ok) break;
-        }
-        // softmax writes P (and has folded the previous O tile) -> O = P . [V_hi | V_lo]
-        ok = mbar_wait(&sm->p_full, j & 1, abort_flag);
-        if (!ok) break;
-        tc_fence_after();
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          const uint32_t v_addr = smem_u32(sm->v[st][ks >> 2]) + 32 * (ks & 3);
-          umma_ts(tmem + kColO, tmem + kColP + 8 * ks, make_desc(v_addr, 1024, kLayoutSw128), idesc_pv, (j | ks) != 0);
+          for (int ks = 0; ks < 8; ++ks) {
+            uint64_t vd;
+            if constexpr (NATURAL) {
+              // 16 keys = two groups of 8 rows of 64 bytes; one swizzle atom spans all 32 dims, so both
+              // strides of the descriptor are the distance between the groups
+              vd = make_desc(smem_u32(sm->v[st][0]) + 1024 * ks, 512, kLayoutSw64);
+              vd = (vd & ~((uint64_t)0x3FFF << 16)) | ((uint64_t)(512 >> 4) << 16);
+            } else {
+              vd = make_desc(smem_u32(sm->v[st][ks >> 2]) + 32 * (ks & 3), 1024, kLayoutSw128);
+            }
+            umma_ts(tmem + kColO, tmem + kColP + 8 * ks, vd, idesc_pv, i > i0 || ks > 0);
+          }
+          umma_commit(&sm->o_full);
+          umma_commit(&sm->kv_empty[st]);
         }
-        umma_commit(&sm->o_full);
-        umma_commit(&sm->kv_empty[st]);
       }
     }
   } else {
@@ -486,23 +597,45 @@ ctx_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     bool ok = true;
     // On an abort the loop still runs every iteration (waits return at once, results are void):
     // both warpgroups must execute the same number of bar.sync instructions.
-    for (int j = 0; j < nt; ++j) {
-      ok = mbar_wait(&sm->s_full, j & 1, abort_flag) && ok;
+    int last = nt - 1;   // number of the last tile walked
+    for (int i = 0; i <= last; ++i) {
+      const int j = i < nt ? i : i - nt;
+      ok = mbar_wait(&sm->s_full, i & 1, abort_flag) && ok;
       tc_fence_after();
       const int n_valid = p.n_ctx - (tile_begin + j) * BN;
-      if (n_valid >= BN)
-        ok = softmax_tile<false>(sm, t_row, wg, row, j & 1, sc, BN, m, l, j == 0, abort_flag) && ok;
-      else
-        ok = softmax_tile<true>(sm, t_row, wg, row, j & 1, sc, n_valid, m, l, j == 0, abort_flag) && ok;
+      if (j == 0 || i >= nt) {
+        if (n_valid >= BN)
+          ok = softmax_tile<false, NATURAL>(sm, t_row, wg, row, i & 1, sc, BN, m, l, j == 0, abort_flag) && ok;
+        else
+          ok = softmax_tile<true, NATURAL>(sm, t_row, wg, row, i & 1, sc, n_valid, m, l, j == 0, abort_flag) && ok;
+      } else {
+        if (n_valid >= BN)
+          ok = softmax_tile_one_pass<false>(sm, t_row, wg, (i & 1) ^ 1, sc, BN, m, l, abort_flag) && ok;
+        else
+          ok = softmax_tile_one_pass<true>(sm, t_row, wg, (i & 1) ^ 1, sc, n_valid, m, l, abort_flag) && ok;
+      }
       tmem_wait_st();
       tc_fence_before();
       mbar_arrive(&sm->p_full);
+      if (i == nt - 1 && nt > 1) {
+        if (!(l < kOnePassMax)) sm->redo = 1;
+        asm volatile("bar.sync 2, 256;" ::: "memory");   // never times out: both warpgroups take the same decision
+        const int redo = *(volatile int*)&sm->redo;
+        mbar_arrive(&sm->verdict);
+        if (redo) {
+          last = 2 * nt - 1;
+          m = -INFINITY;
+          l = 0.f;
+          ok = mbar_wait(&sm->o_full, i & 1, abort_flag) && ok;  // the last P . V has read P
+          tc_fence_after();
+        }
+      }
     }
     if (wg == 1) sm->xsum[row] = l;
     asm volatile("bar.sync 2, 256;" ::: "memory");
     if (wg == 0) {
       l += sm->xsum[row];
-      if (ok) ok = mbar_wait(&sm->o_full, (nt - 1) & 1, abort_flag);
+      if (ok) ok = mbar_wait(&sm->o_full, last & 1, abort_flag);
       if (ok) {
         tc_fence_after();
         float o[DH];
@@ -510,10 +643,12 @@ ctx_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         tmem_wait_ld();
 #pragma unroll
         for (int d = 0; d < DH; ++d) o[d] = __uint_as_float(r[d]);
-        tmem_ld32(t_row + kColO + 32, r);     // P . V_lo
-        tmem_wait_ld();
+        if constexpr (!NATURAL) {
+          tmem_ld32(t_row + kColO + 32, r);     // P . V_lo
+          tmem_wait_ld();
 #pragma unroll
-        for (int d = 0; d < DH; ++d) o[d] += __uint_as_float(r[d]);
+          for (int d = 0; d < DH; ++d) o[d] += __uint_as_float(r[d]);
+        }
         if (row_valid) {
           const float inv = 1.0f / l;
 #pragma unroll
@@ -562,11 +697,11 @@ EncodeTiledFn encode_fn() {
 // descriptors are kept in a small per-thread table, replaced round-robin.
 struct MapKey {
   const void* base;
-  uint64_t inner, outer, row_bytes;
+  uint64_t inner, outer, row_bytes, planes;  // planes > 0: a third dimension of that many [outer][inner] planes
   uint32_t box_inner, box_outer;
   int swz;
   bool operator==(const MapKey& o) const {
-    return base == o.base && inner == o.inner && outer == o.outer && row_bytes == o.row_bytes &&
+    return base == o.base && inner == o.inner && outer == o.outer && row_bytes == o.row_bytes && planes == o.planes &&
            box_inner == o.box_inner && box_outer == o.box_outer && swz == o.swz;
   }
 };
@@ -578,9 +713,9 @@ struct MapCache {
 };
 
 int make_map_2d(CUtensorMap* tm, const void* base, uint64_t inner, uint64_t outer, uint64_t row_bytes, uint32_t box_inner,
-                uint32_t box_outer, CUtensorMapSwizzle swz, const char* what) {
+                uint32_t box_outer, CUtensorMapSwizzle swz, const char* what, uint64_t planes = 0) {
   static thread_local MapCache cache;
-  const MapKey k{base, inner, outer, row_bytes, box_inner, box_outer, (int)swz};
+  const MapKey k{base, inner, outer, row_bytes, planes, box_inner, box_outer, (int)swz};
   for (int i = 0; i < cache.used; ++i)
     if (cache.key[i] == k) {
       *tm = cache.map[i];
@@ -588,11 +723,11 @@ int make_map_2d(CUtensorMap* tm, const void* base, uint64_t inner, uint64_t oute
     }
   EncodeTiledFn fn = encode_fn();
   ARTAB_REQUIRE(fn, ARTAB_EDRIVER, "cuTensorMapEncodeTiled is not available from the driver");
-  const cuuint64_t dims[2] = {inner, outer};
-  const cuuint64_t strides[1] = {row_bytes};
-  const cuuint32_t box[2] = {box_inner, box_outer};
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = fn(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+  const cuuint64_t dims[3] = {inner, outer, planes};
+  const cuuint64_t strides[2] = {row_bytes, outer * row_bytes};
+  const cuuint32_t box[3] = {box_inner, box_outer, 1};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = fn(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, planes ? 3 : 2, const_cast<void*>(base), dims, strides, box, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   ARTAB_REQUIRE(r == CUDA_SUCCESS, ARTAB_EINVAL, "tensor map for %s refused (CUresult %d): base %p, dims %llu x %llu",
@@ -609,9 +744,9 @@ bool ctx_attn_tc_supported(int dtype, int head_dim) { return dtype == ARTAB_BF16
 
 int launch_ctx_attn_tc(const CtxAttnArgs& a, cudaStream_t s) {
   if (a.rows <= 0) return ARTAB_OK;
-  ARTAB_REQUIRE(a.dtype == ARTAB_BF16 && a.head_dim == DH && a.v_transposed, ARTAB_EINVAL,
-                "tensor-core context attention needs bf16, head_dim 32 and a transposed V cache");
-  ARTAB_REQUIRE(a.n_ctx > 0 && a.n_ctx_pad % 8 == 0 && a.n_splits >= 1, ARTAB_EINVAL,
+  ARTAB_REQUIRE(a.dtype == ARTAB_BF16 && a.head_dim == DH && (a.v_transposed || a.n_groups == 1), ARTAB_EINVAL,
+                "tensor-core context attention needs bf16, head_dim 32 and a transposed V cache or one shared context");
+  ARTAB_REQUIRE(a.n_ctx > 0 && (!a.v_transposed || a.n_ctx_pad % 8 == 0) && a.n_splits >= 1, ARTAB_EINVAL,
                 "tensor-core context attention: bad context size");
   ARTAB_REQUIRE(((uintptr_t)a.q % 16) == 0 && ((uintptr_t)a.k_ctx % 16) == 0 && ((uintptr_t)a.v_ctx % 16) == 0,
                 ARTAB_EINVAL, "tensor-core context attention: q / k / v must be 16-byte aligned");
@@ -620,18 +755,25 @@ int launch_ctx_attn_tc(const CtxAttnArgs& a, cudaStream_t s) {
   int rc = make_map_2d(&tq, a.q, (uint64_t)D, (uint64_t)a.rows, (uint64_t)D * 2, DH, BM, CU_TENSOR_MAP_SWIZZLE_64B, "q");
   if (rc) return rc;
   const uint64_t gh = (uint64_t)a.n_groups * a.n_heads;
-  rc = make_map_2d(&tk, a.k_ctx, DH, gh * a.n_ctx_pad, DH * 2, DH, BN, CU_TENSOR_MAP_SWIZZLE_64B, "k_ctx");
-  if (rc) return rc;
-  rc = make_map_2d(&tv, a.v_ctx, (uint64_t)a.n_ctx_pad, gh * 2 * DH, (uint64_t)a.n_ctx_pad * 2, 64, 2 * DH,
-                   CU_TENSOR_MAP_SWIZZLE_128B, "v_ctx");
+  if (a.v_transposed) {
+    rc = make_map_2d(&tk, a.k_ctx, DH, gh * a.n_ctx_pad, DH * 2, DH, BN, CU_TENSOR_MAP_SWIZZLE_64B, "k_ctx");
+    if (rc) return rc;
+    rc = make_map_2d(&tv, a.v_ctx, (uint64_t)a.n_ctx_pad, gh * 2 * DH, (uint64_t)a.n_ctx_pad * 2, 64, 2 * DH,
+                     CU_TENSOR_MAP_SWIZZLE_128B, "v_ctx");
+  } else {
+    rc = make_map_2d(&tk, a.k_ctx, DH, a.n_ctx, DH * 2, DH, BN, CU_TENSOR_MAP_SWIZZLE_64B, "k_ctx", gh);
+    if (rc) return rc;
+    rc = make_map_2d(&tv, a.v_ctx, DH, a.n_ctx, DH * 2, DH, BN, CU_TENSOR_MAP_SWIZZLE_64B, "v_ctx", gh);
+  }
   if (rc) return rc;
 
   // two CTAs per SM at most: each holds 256 of the SM's 512 TMEM columns
   const size_t smem = 100 * 1024;
   static_assert(sizeof(Smem) + 1024 <= 100 * 1024, "shared-memory plan exceeds the request");
-  static SmemConfig configured;
+  static SmemConfig configured[2];
+  auto kernel = a.v_transposed ? ctx_attn_tc_kernel<false> : ctx_attn_tc_kernel<true>;
   {
-    const cudaError_t e = configured.ensure(ctx_attn_tc_kernel, smem, true);
+    const cudaError_t e = configured[a.v_transposed ? 0 : 1].ensure(kernel, smem, true);
     ARTAB_REQUIRE(e == cudaSuccess, ARTAB_ELAUNCH, "ctx_attn_tc_kernel: shared memory refused: %s",
                   cudaGetErrorString(e));
   }
@@ -655,7 +797,7 @@ int launch_ctx_attn_tc(const CtxAttnArgs& a, cudaStream_t s) {
   dim3 grid((rows_in_group + BM - 1) / BM, a.n_heads, a.n_groups * a.n_splits);
   prof_begin(PROF_CTX, s);
   ARTAB_STAMP_ATTACH();
-  const cudaError_t le = launch_dependent(ctx_attn_tc_kernel, grid, dim3(kThreads), smem, s, tq, tk, tv, p);
+  const cudaError_t le = launch_dependent(kernel, grid, dim3(kThreads), smem, s, tq, tk, tv, p);
   prof_end(s);
   ARTAB_REQUIRE(le == cudaSuccess, ARTAB_ELAUNCH, "ctx_attn_tc_kernel: %s", cudaGetErrorString(le));
   count_launch();
