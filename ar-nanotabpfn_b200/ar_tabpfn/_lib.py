@@ -64,6 +64,9 @@ _SIGNATURES = {
                                                 _p]),
     "artab_buffer_attention_merge_visible": (_i, [_i, _p, _p, _i, _i, _i, _i, _i, _p, _i, _p, _p, _p, _i, _i, _p, _p,
                                                   _p]),
+    "artab_hybrid_workspace": (C.c_int64, [_i, _i, _i, _i, _i, _i]),
+    "artab_hybrid_attention": (_i, [_i, _p, _p, _p, _p, _p, _p, C.POINTER(C.c_int64), _i, _i, _i, _i, _i, _i, _p, _p,
+                                    C.c_int64, _p, _p]),
     "artab_kv_append": (_i, [_i, _p, _p, _p, _i, _i, _i, _i, _i, _p]),
     "artab_embed": (_i, [C.POINTER(Model), _p, _p, _p, _i, _i, _i, _p, _p]),
     "artab_head_logpdf": (_i, [C.POINTER(Model), _p, _p, _i, _p, _p]),
@@ -100,11 +103,20 @@ def load_library(path: Optional[str] = None) -> C.CDLL:
     return lib
 
 
+_READY = False
+
+
 def lib() -> C.CDLL:
-    """The loaded library; raises unless a CUDA device is usable."""
+    """The loaded library; raises unless a CUDA device is usable (looked up once: asking the driver costs
+    more than a small call)."""
+    global _READY
+    if _READY and _LIB is not None:
+        return _LIB
     if not torch.cuda.is_available():
         raise RuntimeError("ar_tabpfn (B200 build) needs a CUDA device; there is no CPU fallback")
-    return load_library()
+    handle = load_library()
+    _READY = True
+    return handle
 
 
 class ArtabError(RuntimeError):

@@ -9,6 +9,7 @@ tcgen05 tensor-core kernel (head_dim 32) with fp32 accumulation.
 """
 from __future__ import annotations
 
+import ctypes as C
 from typing import Optional, Tuple
 
 import torch
@@ -27,6 +28,26 @@ def triton_available() -> bool:
         return True
     except Exception:
         return False
+
+
+_STATUS = {}
+
+
+def _status_word(device) -> Tensor:
+    """The device's status word of the calls that do not allocate one each time: zero until a bounded
+    device-side wait gives up (that call's result is NaN); also kept in ``last_status``."""
+    global last_status
+    t = _STATUS.get(device)
+    if t is None:
+        t = _STATUS[device] = torch.zeros(1, device=device, dtype=torch.int32)
+    last_status = t
+    return t
+
+
+def _plain(t: Tensor, dtype) -> Tensor:
+    """``t`` as a contiguous, 16-byte aligned tensor of ``dtype``: itself when it already is one."""
+    t = t.to(dtype).contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
 def _pad8(n: int) -> int:
@@ -263,18 +284,25 @@ def hybrid_attention(q: Tensor, k_ctx: Tensor, v_ctx: Tensor, k_buf: Tensor, v_b
     if Nb == 0:
         return triton_context_attention(q, k_ctx, v_ctx)[0]
     lib = _lib.lib()
-    lens = _stream_lengths(buf_mask, B, H, Lq, Nb, q.device) if buf_mask is not None else None
-    k, v, Nc, Ncp = pack_context(k_ctx.to(q.dtype), v_ctx.to(q.dtype))
-    kv = _pack_buffer(k_buf.to(q.dtype), v_buf.to(q.dtype))
-
-    def context(qr, n):
-        splits = lib.artab_plan_splits(_lib.dtype_code(q.dtype), B * n, n, 1, H, Nc)
-        o, l = _context_partials(qr, k, v, Nc, Ncp, n, splits)
-        return o, l, splits
-
-    if buf_mask is not None and lens is None:
-        return _buffer_merge_masked(q, kv, buf_mask, context, want_lse=False)[0].to(q.dtype)
-    return _buffer_merge(q, kv, lens, context, want_lse=False)[0].to(q.dtype)
+    code = _lib.dtype_code(q.dtype)
+    # token-major queries: with one query per stream that is the tensor itself
+    qr = _plain(q, q.dtype) if Lq == 1 else _rows(q)
+    kc, vc, kb, vb = (_plain(t, q.dtype) for t in (k_ctx, v_ctx, k_buf, v_buf))
+    strides = None
+    if buf_mask is not None:
+        if buf_mask.device != q.device or buf_mask.dtype != torch.bool:
+            buf_mask = buf_mask.to(device=q.device, dtype=torch.bool)
+        buf_mask = buf_mask.expand(B, H, Lq, Nb)
+        strides = (C.c_int64 * 4)(*buf_mask.stride())
+    Nc = kc.shape[1]
+    need = int(lib.artab_hybrid_workspace(code, B, H, Lq, Dh, Nc))
+    ws = torch.empty(need, dtype=torch.uint8, device=q.device)
+    out = torch.empty(B, H, Lq, Dh, dtype=q.dtype, device=q.device)
+    _lib.check(lib.artab_hybrid_attention(
+        code, qr.data_ptr(), kc.data_ptr(), vc.data_ptr(), kb.data_ptr(), vb.data_ptr(), _lib.ptr(buf_mask), strides,
+        B, H, Lq, Dh, Nc, Nb, out.data_ptr(), ws.data_ptr(), need, _status_word(q.device).data_ptr(),
+        _lib.stream_ptr()))
+    return out
 
 
 def hybrid_teacher_forcing_attention(q: Tensor, k_ctx: Tensor, v_ctx: Tensor, k_buf: Tensor, v_buf: Tensor,

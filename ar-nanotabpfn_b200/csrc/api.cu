@@ -889,6 +889,87 @@ int artab_buffer_attention_merge_visible(int dtype, const void* q, const void* k
   return launch_buf_merge(b, (cudaStream_t)stream);
 }
 
+// Key splits of artab_hybrid_attention and where its partials start in the workspace.
+static int hybrid_splits(int dtype, int rows, int n_heads, int head_dim, int n_ctx) {
+  return plan_splits(dtype, head_dim, rows, rows, 1, n_heads, n_ctx, kMaxSplits);
+}
+int64_t artab_hybrid_workspace(int dtype, int n_streams, int n_heads, int n_q, int head_dim, int n_ctx) {
+  const int rows = n_streams * n_q;
+  return (int64_t)hybrid_splits(dtype, rows, n_heads, head_dim, n_ctx) * rows * n_heads * (head_dim + 1) * 4;
+}
+
+int artab_hybrid_attention(int dtype, const void* q, const void* k_ctx, const void* v_ctx, const void* k_buf,
+                           const void* v_buf, const uint8_t* mask, const int64_t* mask_strides, int n_streams,
+                           int n_heads, int n_q, int head_dim, int n_ctx, int n_buf, void* out, void* workspace,
+                           int64_t workspace_bytes, int32_t* status, void* stream) {
+  ARTAB_REQUIRE(q && k_ctx && v_ctx && out && workspace && (n_buf == 0 || (k_buf && v_buf)), ARTAB_EINVAL,
+                "hybrid_attention: null pointer");
+  ARTAB_REQUIRE(dtype == ARTAB_F32 || dtype == ARTAB_BF16, ARTAB_EINVAL, "hybrid_attention: bad dtype %d", dtype);
+  ARTAB_REQUIRE(n_streams >= 0 && n_heads >= 1 && n_q >= 1 && n_ctx >= 1 && n_buf >= 0, ARTAB_EINVAL,
+                "hybrid_attention: bad sizes");
+  ARTAB_REQUIRE(head_dim == 16 || head_dim == 32 || head_dim == 64, ARTAB_EINVAL,
+                "hybrid_attention: head_dim %d not supported (16, 32, 64)", head_dim);
+  ARTAB_REQUIRE(workspace_bytes >= artab_hybrid_workspace(dtype, n_streams, n_heads, n_q, head_dim, n_ctx), ARTAB_ECAPACITY,
+                "hybrid_attention: workspace too small");
+  const uintptr_t bits = (uintptr_t)q | (uintptr_t)k_ctx | (uintptr_t)v_ctx | (uintptr_t)k_buf | (uintptr_t)v_buf |
+                         (uintptr_t)out | (uintptr_t)workspace;
+  ARTAB_REQUIRE(bits % 16 == 0, ARTAB_EINVAL, "hybrid_attention: tensors must be 16-byte aligned");
+  const int rows = n_streams * n_q;
+  if (rows == 0) return ARTAB_OK;
+  cudaStream_t s = (cudaStream_t)stream;
+  CtxAttnArgs c;
+  memset(&c, 0, sizeof(c));
+  c.dtype = dtype;
+  c.q = q;
+  c.k_ctx = k_ctx;
+  c.v_ctx = v_ctx;
+  c.rows = c.rows_per_group = rows;
+  c.n_groups = 1;
+  c.n_heads = n_heads;
+  c.head_dim = head_dim;
+  c.n_ctx = c.n_ctx_pad = n_ctx;
+  c.n_splits = hybrid_splits(dtype, rows, n_heads, head_dim, n_ctx);
+  c.scale = 1.0f / sqrtf((float)head_dim);
+  c.out = (float*)workspace;
+  c.lse = c.out + (size_t)c.n_splits * rows * n_heads * head_dim;
+  c.status = status;
+  int rc;
+  {
+    PlainLaunchScope plain;  // the caller's earlier launches are unknown: see common.cuh
+    rc = use_tc(dtype, head_dim) ? launch_ctx_attn_tc(c, s) : launch_ctx_attn_simt(c, s);
+  }
+  if (rc) return rc;
+  // The merge may start beside the contraction: what it reads before its wait (queries, private K / V, mask)
+  // was complete before the contraction began.
+  BufMergeArgs b;
+  memset(&b, 0, sizeof(b));
+  b.dtype = dtype;
+  b.q = q;
+  b.kv_buf = k_buf;
+  b.v_buf = v_buf;
+  b.n_heads = n_heads;
+  b.head_dim = head_dim;
+  b.max_buf = n_buf;
+  b.op_q = n_q;
+  b.op_out = out;
+  b.key_mask = mask;
+  if (mask) {
+    b.ms_b = mask_strides[0];
+    b.ms_h = mask_strides[1];
+    b.ms_q = mask_strides[2];
+    b.ms_k = mask_strides[3];
+  }
+  const bool pairs = buf_mma_supported(dtype, head_dim);
+  b.n_items = (long)n_streams * n_heads * (pairs ? (n_q + 1) / 2 : n_q);
+  b.o_part = c.out;
+  b.lse_part = c.lse;
+  b.n_splits = c.n_splits;
+  b.rows = rows;
+  b.scale = c.scale;
+  b.poison_if = status;
+  return launch_hybrid_merge(b, s);
+}
+
 int artab_kv_append(int dtype, void* kv_buf, const void* k_new, const void* v_new, int n_streams, int n_heads,
                     int head_dim, int max_buf, int pos, void* stream) {
   PlainLaunchScope plain;  // the caller's earlier launches are unknown: see common.cuh

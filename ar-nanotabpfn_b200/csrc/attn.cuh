@@ -29,6 +29,13 @@ struct BufMergeArgs {
   int tps;                 // mode 2: tokens per stream
   const uint8_t* key_mask; // mode 2, optional: [rows][H][max_buf] bytes, non-zero = the query sees that buffer key
                            // (on top of the visible prefix): arbitrary boolean masks of the functional API
+  // operator form (artab_hybrid_attention): K and V in arrays of their own, [B][H][max_buf][Dh] each; op_q query
+  // rows per stream; key_mask, when given, is addressed with these strides (bytes, 0: broadcast); results
+  // go to op_out as [B][H][op_q][Dh] of the input type
+  const void* v_buf;
+  int op_q;
+  long ms_b, ms_h, ms_q, ms_k;
+  void* op_out;
   const int32_t* lens;     // mode 0: [B] visible buffer rows of each stream, clamped to len0 (null: len0 for all)
   float* lse_out;          // optional [rows][H]: natural-log LSE of the merged attention (-inf: nothing visible)
   long n_items;
@@ -50,6 +57,8 @@ bool ctx_attn_tc_supported(int dtype, int head_dim);
 int launch_buf_merge(const BufMergeArgs& a, cudaStream_t s);      // picks the MMA kernel when it applies
 int launch_buf_merge_mma(const BufMergeArgs& a, cudaStream_t s);  // mma.sync, bf16, head_dim 32
 bool buf_mma_supported(int dtype, int head_dim);
+int launch_hybrid_merge_mma(const BufMergeArgs& a, cudaStream_t s);
+int launch_hybrid_merge(const BufMergeArgs& a, cudaStream_t s);  // operator form of the private-buffer pass
 int launch_kv_append(int dtype, void* kv, const void* k_new, const void* v_new, long n_bh, int dh, int max_buf,
                      int pos, cudaStream_t s);
 

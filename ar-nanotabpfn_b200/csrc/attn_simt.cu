@@ -160,7 +160,7 @@ __device__ __forceinline__ float fast_exp2(float x) {  // MUFU ex2: relative err
 // iteration reads one contiguous span of KPI keys; LPK lanes share a key, each
 // holding one 16-byte slice of the K row and of the V row.
 // ---------------------------------------------------------------------------
-template <typename T, int DH>
+template <typename T, int DH, bool OP>   // OP: the operator form, see buf_mma_kernel; one query row per item
 __global__ void __launch_bounds__(128, 6) buf_merge_kernel(const BufMergeArgs a) {
   dep_trigger();  // the dependent dense chain reads only model constants before its wait (see buf_mma_kernel)
   constexpr int VEC = Vec16<T>::N;
@@ -176,7 +176,17 @@ __global__ void __launch_bounds__(128, 6) buf_merge_kernel(const BufMergeArgs a)
   int h, len;
   long row_t, row_b;
   const uint8_t* mrow = nullptr;  // optional per-key visibility of this item's query (mode 2)
-  if (a.mode_tf == 2) {
+  [[maybe_unused]] int oq = 0;
+  if constexpr (OP) {
+    oq = (int)(item % a.op_q);
+    const long bh = item / a.op_q;
+    b = bh / a.n_heads;
+    h = (int)(bh - b * a.n_heads);
+    len = a.max_buf;
+    row_t = b * a.op_q + oq;
+    row_b = -1;
+    if (a.key_mask) mrow = a.key_mask + b * a.ms_b + h * a.ms_h + oq * a.ms_q;
+  } else if (a.mode_tf == 2) {
     // one query per item: token j of stream b sees the first visible[j] buffer rows
     const int j = (int)(item % a.tps);
     const long bh = item / a.tps;
@@ -225,7 +235,8 @@ __global__ void __launch_bounds__(128, 6) buf_merge_kernel(const BufMergeArgs a)
 #pragma unroll
     for (int e = 0; e < VEC; ++e) acc[w][e] = 0.f;
 
-  const T* kv = reinterpret_cast<const T*>(a.kv_buf) + ((size_t)(b * a.n_heads + h) * a.max_buf) * 2 * DH;
+  const T* kv = reinterpret_cast<const T*>(a.kv_buf) + ((size_t)(b * a.n_heads + h) * a.max_buf) * (OP ? 1 : 2) * DH;
+  const T* vv = OP ? reinterpret_cast<const T*>(a.v_buf) + ((size_t)(b * a.n_heads + h) * a.max_buf) * DH : kv + DH;
   // Keys are walked in chunks of CH warp iterations: all 2*CH 16-byte loads of a chunk are issued
   // before the first is used, so a warp has CH KiB in flight and pays one memory round trip per
   // chunk instead of one per iteration.
@@ -236,9 +247,9 @@ __global__ void __launch_bounds__(128, 6) buf_merge_kernel(const BufMergeArgs a)
     for (int c = 0; c < CH; ++c) {
       const int key = key0 + c * KPI + grp;
       if (key < len) {
-        const uint4* p = reinterpret_cast<const uint4*>(kv + (size_t)key * 2 * DH + sub * VEC);
-        kr[c] = __ldg(p);
-        vr[c] = __ldg(p + LPK);  // the V row follows the K row: DH elements = LPK 16-byte slices
+        const size_t at = (size_t)key * (OP ? 1 : 2) * DH + sub * VEC;
+        kr[c] = __ldg(reinterpret_cast<const uint4*>(kv + at));
+        vr[c] = __ldg(reinterpret_cast<const uint4*>(vv + at));
       } else {
         kr[c] = make_uint4(0u, 0u, 0u, 0u);
         vr[c] = kr[c];
@@ -264,7 +275,7 @@ __global__ void __launch_bounds__(128, 6) buf_merge_kernel(const BufMergeArgs a)
         s1 += __shfl_xor_sync(0xffffffffu, s1, o);
       }
       bool valid = key0 + c * KPI + grp < len;
-      if (valid && mrow) valid = mrow[key0 + c * KPI + grp] != 0;
+      if (valid && mrow) valid = mrow[(OP ? a.ms_k : 1L) * (key0 + c * KPI + grp)] != 0;
       sc0[c] = valid ? s0 : -INFINITY;
       sc1[c] = valid ? s1 : -INFINITY;
     }
@@ -368,11 +379,17 @@ __global__ void __launch_bounds__(128, 6) buf_merge_kernel(const BufMergeArgs a)
     if (grp == 0) {
       float inv = wsum > 0.f ? 1.0f / wsum : 0.f;
       if (a.poison_if && __ldcg(a.poison_if) != 0) inv = __int_as_float(0x7fc00000);
+      if constexpr (OP) {
+        T* dst = reinterpret_cast<T*>(a.op_out) + ((size_t)(b * a.n_heads + h) * a.op_q + oq) * DH + sub * VEC;
 #pragma unroll
-      for (int e = 0; e < VEC; e += 4) {
-        float* dst = a.out + (a.out_lane_major ? lane_major_index(r, h * DH + sub * VEC + e, a.n_heads * DH)
-                                               : ((size_t)r * a.n_heads + h) * DH + sub * VEC + e);
-        *reinterpret_cast<float4*>(dst) = make_float4(o[e] * inv, o[e + 1] * inv, o[e + 2] * inv, o[e + 3] * inv);
+        for (int e = 0; e < VEC; ++e) dst[e] = from_f32<T>(o[e] * inv);
+      } else {
+#pragma unroll
+        for (int e = 0; e < VEC; e += 4) {
+          float* dst = a.out + (a.out_lane_major ? lane_major_index(r, h * DH + sub * VEC + e, a.n_heads * DH)
+                                                 : ((size_t)r * a.n_heads + h) * DH + sub * VEC + e);
+          *reinterpret_cast<float4*>(dst) = make_float4(o[e] * inv, o[e + 1] * inv, o[e + 2] * inv, o[e + 3] * inv);
+        }
       }
     }
   }
@@ -406,7 +423,7 @@ int launch_ctx_t(const CtxAttnArgs& a, cudaStream_t s) {
   return check_launch("ctx_attn_simt_kernel");
 }
 
-template <typename T>
+template <typename T, bool OP>
 int launch_buf_t(const BufMergeArgs& a, cudaStream_t s) {
   const int wpb = 4;
   const unsigned grid = (unsigned)((a.n_items + wpb - 1) / wpb);
@@ -415,9 +432,9 @@ int launch_buf_t(const BufMergeArgs& a, cudaStream_t s) {
                 "buffer attention: head_dim %d not supported (16, 32, 64)", a.head_dim);
   prof_begin(PROF_BUF, s);
   switch (a.head_dim) {
-    case 16: le = launch_dependent(buf_merge_kernel<T, 16>, dim3(grid), dim3(wpb * 32), 0, s, a); break;
-    case 32: le = launch_dependent(buf_merge_kernel<T, 32>, dim3(grid), dim3(wpb * 32), 0, s, a); break;
-    default: le = launch_dependent(buf_merge_kernel<T, 64>, dim3(grid), dim3(wpb * 32), 0, s, a); break;
+    case 16: le = launch_dependent(buf_merge_kernel<T, 16, OP>, dim3(grid), dim3(wpb * 32), 0, s, a); break;
+    case 32: le = launch_dependent(buf_merge_kernel<T, 32, OP>, dim3(grid), dim3(wpb * 32), 0, s, a); break;
+    default: le = launch_dependent(buf_merge_kernel<T, 64, OP>, dim3(grid), dim3(wpb * 32), 0, s, a); break;
   }
   prof_end(s);
   ARTAB_REQUIRE(le == cudaSuccess, ARTAB_ELAUNCH, "buf_merge_kernel: %s", cudaGetErrorString(le));
@@ -436,7 +453,13 @@ int launch_ctx_attn_simt(const CtxAttnArgs& a, cudaStream_t s) {
 int launch_buf_merge(const BufMergeArgs& a, cudaStream_t s) {
   if (a.n_items <= 0) return ARTAB_OK;
   if (a.mode_tf != 2 && buf_mma_supported(a.dtype, a.head_dim)) return launch_buf_merge_mma(a, s);
-  return a.dtype == ARTAB_BF16 ? launch_buf_t<__nv_bfloat16>(a, s) : launch_buf_t<float>(a, s);
+  return a.dtype == ARTAB_BF16 ? launch_buf_t<__nv_bfloat16, false>(a, s) : launch_buf_t<float, false>(a, s);
+}
+
+int launch_hybrid_merge(const BufMergeArgs& a, cudaStream_t s) {
+  if (a.n_items <= 0) return ARTAB_OK;
+  if (buf_mma_supported(a.dtype, a.head_dim)) return launch_hybrid_merge_mma(a, s);
+  return a.dtype == ARTAB_BF16 ? launch_buf_t<__nv_bfloat16, true>(a, s) : launch_buf_t<float, true>(a, s);
 }
 
 int launch_kv_append(int dtype, void* kv, const void* k_new, const void* v_new, long n_bh, int dh, int max_buf,

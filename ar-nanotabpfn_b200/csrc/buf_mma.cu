@@ -61,6 +61,10 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// OP: the operator form.  K rows and V rows come from two arrays, an item is a pair of query rows of one
+// (stream, head), any boolean mask is looked up key by key, the result is stored in bf16 where the caller
+// wants it: nothing has to be packed, measured (mask -> lengths) or converted around the launch.
+template <bool OP>
 __global__ void __launch_bounds__(WPB * 32, 6) buf_mma_kernel(const BufMergeArgs a) {
   __shared__ __align__(16) uint8_t vs[WPB][NR][KB * PITCH];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -76,9 +80,18 @@ __global__ void __launch_bounds__(WPB * 32, 6) buf_mma_kernel(const BufMergeArgs
   const int t4 = lane & 3;   // fragment column pair
 
   long b;
-  int h, len;
+  int h, len, q0 = 0;
   long rows2[2];
-  if (a.mode_tf) {
+  if constexpr (OP) {
+    const int pairs = (a.op_q + 1) >> 1;
+    const long bh = item / pairs;
+    q0 = 2 * (int)(item - bh * pairs);
+    b = bh / a.n_heads;
+    h = (int)(bh - b * a.n_heads);
+    len = a.max_buf;
+    rows2[0] = b * a.op_q + q0;
+    rows2[1] = q0 + 1 < a.op_q ? rows2[0] + 1 : -1;
+  } else if (a.mode_tf) {
     const int ips = a.nt + 1;
     const int i = (int)(item % ips);
     const long bh = item / ips;
@@ -106,8 +119,14 @@ __global__ void __launch_bounds__(WPB * 32, 6) buf_mma_kernel(const BufMergeArgs
       qa[ks][1] = __ldg(qp + 8 * ks + 4);
     }
   }
-  const __nv_bfloat16* kv =
-      reinterpret_cast<const __nv_bfloat16*>(a.kv_buf) + ((size_t)(b * a.n_heads + h) * a.max_buf) * 2 * DH;
+  const __nv_bfloat16* kv = reinterpret_cast<const __nv_bfloat16*>(a.kv_buf) +
+                            ((size_t)(b * a.n_heads + h) * a.max_buf) * (OP ? 1 : 2) * DH;
+  [[maybe_unused]] const __nv_bfloat16* vsep = nullptr;
+  [[maybe_unused]] const uint8_t* mrow = nullptr;  // mask bytes of this lane's query row
+  if constexpr (OP) {
+    vsep = reinterpret_cast<const __nv_bfloat16*>(a.v_buf) + ((size_t)(b * a.n_heads + h) * a.max_buf) * DH;
+    if (a.key_mask && g < 2 && rows2[g] >= 0) mrow = a.key_mask + b * a.ms_b + h * a.ms_h + (q0 + g) * a.ms_q;
+  }
   const float sc = a.scale * kLog2e;
   const int nblk = (len + KB - 1) / KB;
 
@@ -121,7 +140,11 @@ __global__ void __launch_bounds__(WPB * 32, 6) buf_mma_kernel(const BufMergeArgs
         const int c = i * 32 + lane, key = c >> 3, part = c & 7;
         const int gkey = kb * KB + key;
         const bool valid = gkey < len;
-        const __nv_bfloat16* src = kv + (valid ? ((size_t)gkey * 2 * DH + part * 8) : 0);
+        const __nv_bfloat16* src;
+        if constexpr (OP)
+          src = (part < 4 ? kv : vsep) + (valid ? (size_t)gkey * DH + (part & 3) * 8 : 0);
+        else
+          src = kv + (valid ? ((size_t)gkey * 2 * DH + part * 8) : 0);
         cp_async16(vs_base + (uint32_t)((kb % NR) * (KB * PITCH) + key * PITCH + part * 16), src, valid);
       }
     }
@@ -163,15 +186,20 @@ __global__ void __launch_bounds__(WPB * 32, 6) buf_mma_kernel(const BufMergeArgs
 #pragma unroll
     for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-      for (int e = 0; e < 2; ++e) sv[nt * 2 + e] = key0 + nt * 8 + e < len ? s[nt][e] * sc : -INFINITY;
+      for (int e = 0; e < 2; ++e) {
+        bool vis = key0 + nt * 8 + e < len;
+        if constexpr (OP) vis = vis && (!mrow || mrow[(long)(key0 + nt * 8 + e) * a.ms_k] != 0);
+        sv[nt * 2 + e] = vis ? s[nt][e] * sc : -INFINITY;
+      }
     float bm = fmaxf(fmaxf(sv[0], sv[1]), fmaxf(sv[2], sv[3]));
     bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 1));
-    bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 2));   // finite: key kb*16 of every block is valid
+    bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 2));   // finite without a mask: key kb*16 of every block is valid
     const float m_new = fmaxf(m, bm);
-    const float alpha = fast_exp2(m - m_new);              // first block: exp2(-inf) = 0
+    const float ref = OP && m_new == -INFINITY ? 0.f : m_new;  // nothing visible yet: exp2(-inf - 0) = 0
+    const float alpha = fast_exp2(m - ref);                // first block: exp2(-inf) = 0
     float p[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) p[i] = fast_exp2(sv[i] - m_new);
+    for (int i = 0; i < 4; ++i) p[i] = fast_exp2(sv[i] - ref);
     l = l * alpha + (p[0] + p[1]) + (p[2] + p[3]);         // this lane's share of the row sum
     m = m_new;
 #pragma unroll
@@ -259,11 +287,18 @@ __global__ void __launch_bounds__(WPB * 32, 6) buf_mma_kernel(const BufMergeArgs
   if (a.lse_out && t4 == 0) a.lse_out[(size_t)r * a.n_heads + h] = wsum > 0.f ? top + logf(wsum) : -INFINITY;
   float inv = wsum > 0.f ? 1.0f / wsum : 0.f;
   if (a.poison_if && __ldcg(a.poison_if) != 0) inv = __int_as_float(0x7fc00000);
+  if constexpr (OP) {
+    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.op_out) + ((size_t)(b * a.n_heads + h) * a.op_q + q0 + g) * DH + t4 * 2;
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const int col = h * DH + 8 * j + t4 * 2;
-    float* dst = a.out + (a.out_lane_major ? lane_major_index(r, col, a.n_heads * DH) : (size_t)r * a.n_heads * DH + col);
-    *reinterpret_cast<float2*>(dst) = make_float2(out[2 * j] * inv, out[2 * j + 1] * inv);
+    for (int j = 0; j < 4; ++j)
+      *reinterpret_cast<uint32_t*>(dst + 8 * j) = pack_bf16(out[2 * j] * inv, out[2 * j + 1] * inv);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int col = h * DH + 8 * j + t4 * 2;
+      float* dst = a.out + (a.out_lane_major ? lane_major_index(r, col, a.n_heads * DH) : (size_t)r * a.n_heads * DH + col);
+      *reinterpret_cast<float2*>(dst) = make_float2(out[2 * j] * inv, out[2 * j + 1] * inv);
+    }
   }
   if (threadIdx.x == 0) ARTAB_STAMP(3, 2);
 }
@@ -515,8 +550,18 @@ int launch_buf_merge_mma(const BufMergeArgs& a, cudaStream_t s) {
     le = launch_dependent(buf_mma_tf_kernel, dim3(grid), dim3(WPB * 32), 0, s, a, n_groups);
   } else {
     const unsigned grid = (unsigned)((a.n_items + WPB - 1) / WPB);
-    le = launch_dependent(buf_mma_kernel, dim3(grid), dim3(WPB * 32), 0, s, a);
+    le = launch_dependent(buf_mma_kernel<false>, dim3(grid), dim3(WPB * 32), 0, s, a);
   }
+  prof_end(s);
+  ARTAB_REQUIRE(le == cudaSuccess, ARTAB_ELAUNCH, "buf_mma_kernel: %s", cudaGetErrorString(le));
+  count_launch();
+  return check_launch("buf_mma_kernel");
+}
+
+int launch_hybrid_merge_mma(const BufMergeArgs& a, cudaStream_t s) {
+  prof_begin(PROF_BUF, s);
+  const unsigned grid = (unsigned)((a.n_items + WPB - 1) / WPB);
+  const cudaError_t le = launch_dependent(buf_mma_kernel<true>, dim3(grid), dim3(WPB * 32), 0, s, a);
   prof_end(s);
   ARTAB_REQUIRE(le == cudaSuccess, ARTAB_ELAUNCH, "buf_mma_kernel: %s", cudaGetErrorString(le));
   count_launch();

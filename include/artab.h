@@ -324,6 +324,19 @@ ARTAB_API int artab_buffer_attention_merge_ragged(int dtype, const void* q, cons
                                         int len_max, const float* o_part, const float* lse_part, int n_splits,
                                         int rows, float* out, float* lse_out, void* stream);
 
+/* Decode attention of the functional API in two launches on the caller's own tensors, nothing packed or
+ * measured in between: shared context and private buffers merged by log-sum-exp.
+ *   q [B*Lq][H][Dh] (token-major; the reference's [B,H,1,Dh] as it is when Lq = 1); k_ctx / v_ctx [H][Nc][Dh];
+ *   k_buf / v_buf [B][H][Nb][Dh]; mask: one byte per key, non-zero = visible, element (b, h, l, key) at
+ *   mask + sum of index * mask_strides[i] (HOST array of four, 0 broadcasts), or NULL: every key visible;
+ *   out [B][H][Lq][Dh] of the input type; workspace of artab_hybrid_workspace bytes.
+ * Replaces hybrid_attention (ar_tabpfn/model/triton_kernels.py:662-708). */
+ARTAB_API int64_t artab_hybrid_workspace(int dtype, int n_streams, int n_heads, int n_q, int head_dim, int n_ctx);
+ARTAB_API int artab_hybrid_attention(int dtype, const void* q, const void* k_ctx, const void* v_ctx, const void* k_buf,
+                           const void* v_buf, const uint8_t* mask, const int64_t* mask_strides, int n_streams,
+                           int n_heads, int n_q, int head_dim, int n_ctx, int n_buf, void* out, void* workspace,
+                           int64_t workspace_bytes, int32_t* status, void* stream);
+
 /* In-place append of one new K/V row per (stream, head) at position `pos`.
  *   k_new, v_new [B][H][Dh] (dtype).
  * Replaces the slice assignment into k_buf_cache / v_buf_cache

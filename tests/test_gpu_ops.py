@@ -335,3 +335,36 @@ def test_decode_attention_microbenchmark_shapes_bf16(tk):
     rel = (got - want).norm(dim=-1) / want.norm(dim=-1).clamp_min(1e-6)
     assert rel.max() <= 1e-2, rel.max()
     assert (lens == 0).any() and (lens == Nb).any()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape", [(1, 2, 1, 32, 1, 1), (37, 4, 1, 32, 127, 15), (130, 3, 1, 32, 129, 17), (5, 2, 3, 32, 300, 33),
+                                   (9, 4, 2, 16, 70, 16), (6, 2, 1, 64, 65, 20), (700, 4, 1, 32, 2048, 40)],
+                         ids=lambda s: "b%d_h%d_q%d_d%d_nc%d_nb%d" % s)
+def test_hybrid_attention_masks_and_tile_edges(shape, dtype):
+    """The two-launch operator on the caller's tensors: key tiles of 128 and 64, private blocks of 16, query pairs,
+    every way a mask broadcasts, rows that see no private key, tensors that are views off a 16-byte boundary."""
+    from ar_tabpfn.model import triton_kernels as tk
+    from util import ref_attention
+    B, H, Lq, Dh, Nc, Nb = shape
+    g = torch.Generator(device="cuda").manual_seed(B + Nc)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).to(dtype)
+    q, kc, vc = r(B, H, Lq, Dh), r(H, Nc, Dh), r(H, Nc, Dh)
+    kb, vb = (r(B * H * Nb * Dh + 1)[1:].view(B, H, Nb, Dh) for _ in range(2))
+    lens = torch.randint(0, Nb + 1, (B,), device="cuda", generator=g)
+    prefix = (torch.arange(Nb, device="cuda")[None] < lens[:, None]).view(B, 1, 1, Nb)
+    masks = [None, prefix, torch.rand(B, H, Lq, Nb, device="cuda", generator=g) < 0.5,
+             torch.rand(1, 1, Lq, Nb, device="cuda", generator=g) < 0.5, torch.zeros(B, 1, 1, 1, dtype=torch.bool, device="cuda")]
+    for m in masks:
+        got = tk.hybrid_attention(q, kc, vc, kb, vb, buf_mask=m)
+        assert got.shape == q.shape and got.dtype == dtype and int(tk.last_status.item()) == 0
+        k = torch.cat([kc.expand(B, -1, -1, -1), kb], dim=2)
+        v = torch.cat([vc.expand(B, -1, -1, -1), vb], dim=2)
+        full = torch.ones(B, H, Lq, Nc + Nb, dtype=torch.bool, device="cuda")
+        if m is not None:
+            full[..., Nc:] = m
+        want = ref_attention(q, k, v, full)[0]
+        # bf16: softmax numerators of the context and the result are rounded to 8 bits (2^-9 each, the first
+        # averaged over the keys); fp32: sums over up to 2088 keys
+        rel = float((got.float() - want).norm() / want.norm())
+        assert rel <= (2 ** -8 if dtype == torch.bfloat16 else 1e-5), rel
