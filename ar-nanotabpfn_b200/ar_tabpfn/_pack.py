@@ -129,7 +129,7 @@ class PackedModel:
         self._layers = (_lib.LayerWeights * self.n_layers)()
         for i in range(self.n_layers):
             for f, _ in _lib.LayerWeights._fields_:
-                if not f.startswith("tc_"):
+                if not f.startswith(("tc_", "fma_")):
                     setattr(self._layers[i], f, P(f"{i}.{f}"))
         m = _lib.Model()
         m.d_model, m.n_heads, m.head_dim, m.d_ff = self.d_model, self.n_heads, self.head_dim, self.d_ff
@@ -141,6 +141,7 @@ class PackedModel:
         self.struct = m
         self._pack_tensor_core(embedder, backbone, head, target)
         self._pack_sequence(dict(items), target)
+        self._pack_panels(dict(items), target)
 
     def _pack_tensor_core(self, embedder, backbone, head, target):
         """bf16 hi/lo tiles for the tcgen05 per-token chain (d_model in {64,128,192}, d_ff % 128 == 0,
@@ -244,6 +245,30 @@ class PackedModel:
         self.struct.seq_rank_bytes = 4 * flat.shape[1]
         self.seq_flat = flat.to(target)
         self.struct.seq_w = self.seq_flat.data_ptr()
+
+    def _pack_panels(self, w, target):
+        """D x D panels of every matrix for the register-tiled fp32 chain, in the order it uses them."""
+        D, Dff, K = self.d_model, self.d_ff, self.n_comp
+        self.fma_flat = None
+        if D not in (64, 128, 192) or Dff % D or Dff > 1024 or 3 * K > D:
+            return
+        chunks = range(0, Dff, D)
+        wb = torch.zeros(Dff, D, dtype=torch.float64)
+        wb[:, :3 * K] = w["wb_t"]
+        stacks = []
+        for i in range(self.n_layers):
+            stacks.append([w[f"{i}.wf_t"], *w[f"{i}.wqkv_t"].split(D, dim=1)])
+            stacks.append([w[f"{i}.wo_t"]] + [p for j in chunks for p in (w[f"{i}.w1_t"][:, j:j + D], w[f"{i}.w2_t"][j:j + D])])
+        stacks.append([p for j in chunks for p in (w["wa_t"][:, j:j + D], wb[j:j + D])])
+        flat = torch.cat([p.reshape(-1).to(torch.float32) for st in stacks for p in st]).to(target)
+        self.fma_flat = flat
+        at = flat.data_ptr()
+        for n, st in enumerate(stacks):
+            if n == len(stacks) - 1:
+                self.struct.fma_head = at
+            else:
+                setattr(self._layers[n // 2], ("fma_pre", "fma_post")[n % 2], at)
+            at += 4 * D * D * len(st)
 
     @property
     def ref(self):

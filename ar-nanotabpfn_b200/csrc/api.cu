@@ -158,12 +158,11 @@ bool use_tc(int dtype, int head_dim) { return ctx_attn_tc_supported(dtype, head_
 int plan_splits(int dtype, int head_dim, int rows, int rows_per_group, int n_groups, int n_heads, int n_ctx,
                 int max_splits) {
   const bool tc = use_tc(dtype, head_dim);
-  const int tile_m = tc ? 128 : 16, tile_k = tc ? 128 : 64;
   const int rows_g = n_groups == 1 ? rows : rows_per_group;
+  const int tile_m = tc ? 128 : ctx_attn_fma_rows(rows_g), tile_k = tc ? 128 : 64;
   const long items = (long)((rows_g + tile_m - 1) / tile_m) * n_heads * n_groups;
   const int tiles = (n_ctx + tile_k - 1) / tile_k;
-  // Resident CTA slots: two per SM for the tensor-core kernel (TMEM), about eight for the SIMT one.
-  const long slots = (long)kSMs * (tc ? 2 : 8);
+  const long slots = (long)kSMs * 2;   // resident CTAs: two per SM (tensor memory / registers)
   // Cost model: waves x (key tiles per CTA + fixed per-CTA overhead in tile units); smallest wins.
   int best = 1;
   double best_cost = 1e30;
@@ -222,6 +221,7 @@ void fill_head(const artab_model* m, DenseArgs& d) {
   d.tc_wa = m->tc_wa;
   d.tc_wb = m->tc_wb;
   d.tc_head_lo = m->tc_head_lo;
+  d.fma_head = m->fma_head;
 }
 
 DenseArgs dense_base(const artab_model* m, const artab_state* st, int rows) {

@@ -1,9 +1,5 @@
-// SIMT attention kernels.
+// SIMT kernels of the private buffers.
 //
-//  * ctx_attn_simt_kernel  — queries of many streams against one shared (or one
-//    per-group) context K/V with online softmax and LSE output; fp32 FMA math.
-//    This is the context kernel of the fp32 mode (and of head sizes the
-//    tensor-core kernel is not built for).
 //  * buf_merge_kernel      — the bandwidth-bound warp-level pass over each
 //    stream's private buffer K/V, merged in registers by log-sum-exp with the
 //    context partials (any number of key splits).  Used by both dtypes.
@@ -13,140 +9,6 @@
 namespace artab {
 
 namespace {
-
-constexpr int kQW = 4;        // queries per warp
-constexpr int kWarps = 4;     // warps per CTA
-constexpr int kQB = kQW * kWarps;
-constexpr int kKT = 64;       // keys per tile
-
-template <typename T, int DH>
-__global__ void __launch_bounds__(kWarps * 32) ctx_attn_simt_kernel(const CtxAttnArgs a) {
-  constexpr int NDL = DH >= 32 ? DH / 32 : 1;  // output dims per lane
-  __shared__ float sK[kKT][DH + 1];
-  __shared__ float sV[kKT][DH];
-  __shared__ float sQ[kQB][DH];
-  __shared__ __align__(16) float sP[kWarps][kKT][kQW];
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int h = blockIdx.y;
-  const int g = blockIdx.z / a.n_splits, split = blockIdx.z - g * a.n_splits;
-  const int rows_in_group = a.n_groups == 1 ? a.rows : a.rows_per_group;
-  const long group_row0 = a.n_groups == 1 ? 0 : (long)g * a.rows_per_group;
-  const int q0 = blockIdx.x * kQB;
-  if (q0 >= rows_in_group) return;
-
-  const int tiles = (a.n_ctx + kKT - 1) / kKT;
-  const int tps = (tiles + a.n_splits - 1) / a.n_splits;
-  const int k_begin = split * tps * kKT;
-  const int k_end = min(a.n_ctx, k_begin + tps * kKT);
-
-  const T* Q = reinterpret_cast<const T*>(a.q);
-  const T* Kc = reinterpret_cast<const T*>(a.k_ctx) + ((size_t)(g * a.n_heads + h) * a.n_ctx_pad) * DH;
-  // transposed layout holds a hi and a lo part per head: [2*Dh][Ncp]
-  const T* Vc = reinterpret_cast<const T*>(a.v_ctx) +
-                ((size_t)(g * a.n_heads + h) * a.n_ctx_pad) * DH * (a.v_transposed ? 2 : 1);
-
-  for (int i = threadIdx.x; i < kQB * DH; i += blockDim.x) {
-    const int qi = i / DH, d = i - qi * DH;
-    const int r = q0 + qi;
-    sQ[qi][d] = r < rows_in_group ? to_f32<T>(Q[((size_t)(group_row0 + r) * a.n_heads + h) * DH + d]) : 0.f;
-  }
-
-  float m[kQW], l[kQW], acc[kQW][NDL];
-#pragma unroll
-  for (int qq = 0; qq < kQW; ++qq) {
-    m[qq] = -INFINITY;
-    l[qq] = 0.f;
-#pragma unroll
-    for (int e = 0; e < NDL; ++e) acc[qq][e] = 0.f;
-  }
-  const float sc = a.scale * kLog2e;
-
-  for (int kt = k_begin; kt < k_end; kt += kKT) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < kKT * DH; i += blockDim.x) {
-      const int key = i / DH, d = i - key * DH;
-      sK[key][d] = (kt + key) < a.n_ctx ? to_f32<T>(Kc[(size_t)(kt + key) * DH + d]) : 0.f;
-    }
-    if (a.v_transposed) {
-      for (int i = threadIdx.x; i < kKT * DH; i += blockDim.x) {
-        const int d = i / kKT, key = i - d * kKT;
-        sV[key][d] = (kt + key) < a.n_ctx ? to_f32<T>(Vc[(size_t)d * a.n_ctx_pad + kt + key]) +
-                                                 to_f32<T>(Vc[(size_t)(DH + d) * a.n_ctx_pad + kt + key])
-                                           : 0.f;
-      }
-    } else {
-      for (int i = threadIdx.x; i < kKT * DH; i += blockDim.x) {
-        const int key = i / DH, d = i - key * DH;
-        sV[key][d] = (kt + key) < a.n_ctx ? to_f32<T>(Vc[(size_t)(kt + key) * DH + d]) : 0.f;
-      }
-    }
-    __syncthreads();
-
-    float s0[kQW], s1[kQW];
-#pragma unroll
-    for (int qq = 0; qq < kQW; ++qq) s0[qq] = s1[qq] = 0.f;
-#pragma unroll 8
-    for (int d = 0; d < DH; ++d) {
-      const float k0 = sK[lane][d], k1 = sK[lane + 32][d];
-#pragma unroll
-      for (int qq = 0; qq < kQW; ++qq) {
-        const float qv = sQ[warp * kQW + qq][d];
-        s0[qq] = fmaf(qv, k0, s0[qq]);
-        s1[qq] = fmaf(qv, k1, s1[qq]);
-      }
-    }
-    const bool v0 = kt + lane < k_end, v1 = kt + lane + 32 < k_end;
-#pragma unroll
-    for (int qq = 0; qq < kQW; ++qq) {
-      const float a0 = v0 ? s0[qq] * sc : -INFINITY;
-      const float a1 = v1 ? s1[qq] * sc : -INFINITY;
-      const float mn = fmaxf(m[qq], warp_max(fmaxf(a0, a1)));  // finite: every tile holds a valid key
-      const float alpha = exp2f(m[qq] - mn);
-      const float p0 = exp2f(a0 - mn), p1 = exp2f(a1 - mn);
-      l[qq] = l[qq] * alpha + warp_sum(p0 + p1);
-      m[qq] = mn;
-#pragma unroll
-      for (int e = 0; e < NDL; ++e) acc[qq][e] *= alpha;
-      sP[warp][lane][qq] = p0;
-      sP[warp][lane + 32][qq] = p1;
-    }
-    __syncwarp();
-    if (DH >= 32 || lane < DH) {
-#pragma unroll 4
-      for (int key = 0; key < kKT; ++key) {
-        const float4 p4 = *reinterpret_cast<const float4*>(&sP[warp][key][0]);
-#pragma unroll
-        for (int e = 0; e < NDL; ++e) {
-          const float v = sV[key][lane + 32 * e];
-          acc[0][e] = fmaf(p4.x, v, acc[0][e]);
-          acc[1][e] = fmaf(p4.y, v, acc[1][e]);
-          acc[2][e] = fmaf(p4.z, v, acc[2][e]);
-          acc[3][e] = fmaf(p4.w, v, acc[3][e]);
-        }
-      }
-    }
-    __syncwarp();
-  }
-
-#pragma unroll
-  for (int qq = 0; qq < kQW; ++qq) {
-    const int r = q0 + warp * kQW + qq;
-    if (r >= rows_in_group) continue;
-    const size_t ro = ((size_t)split * a.rows + group_row0 + r) * a.n_heads + h;
-    const float inv = l[qq] > 0.f ? 1.0f / l[qq] : 0.f;
-    if (DH >= 32 || lane < DH) {
-#pragma unroll
-      for (int e = 0; e < NDL; ++e) {
-        const size_t idx = a.out_lane_major
-                               ? lane_major_index(group_row0 + r, h * DH + lane + 32 * e, a.n_heads * DH)
-                               : ro * DH + lane + 32 * e;
-        a.out[idx] = acc[qq][e] * inv;
-      }
-    }
-    if (lane == 0) a.lse[ro] = l[qq] > 0.f ? (m[qq] + log2f(l[qq])) * kLn2 : -INFINITY;
-  }
-}
 
 __device__ __forceinline__ float fast_exp2(float x) {  // MUFU ex2: relative error 2^-22, exp2(-inf) = 0
   float y;
@@ -406,23 +268,6 @@ __global__ void kv_append_kernel(T* kv, const T* k_new, const T* v_new, long n_b
   p[dh] = v_new[i];
 }
 
-template <typename T>
-int launch_ctx_t(const CtxAttnArgs& a, cudaStream_t s) {
-  const int rows_in_group = a.n_groups == 1 ? a.rows : a.rows_per_group;
-  dim3 grid((rows_in_group + kQB - 1) / kQB, a.n_heads, a.n_groups * a.n_splits);
-  ARTAB_REQUIRE(a.head_dim == 16 || a.head_dim == 32 || a.head_dim == 64, ARTAB_EINVAL,
-                "context attention: head_dim %d not supported (16, 32, 64)", a.head_dim);
-  prof_begin(PROF_CTX, s);
-  switch (a.head_dim) {
-    case 16: ctx_attn_simt_kernel<T, 16><<<grid, kWarps * 32, 0, s>>>(a); break;
-    case 32: ctx_attn_simt_kernel<T, 32><<<grid, kWarps * 32, 0, s>>>(a); break;
-    default: ctx_attn_simt_kernel<T, 64><<<grid, kWarps * 32, 0, s>>>(a); break;
-  }
-  prof_end(s);
-  count_launch();
-  return check_launch("ctx_attn_simt_kernel");
-}
-
 template <typename T, bool OP>
 int launch_buf_t(const BufMergeArgs& a, cudaStream_t s) {
   const int wpb = 4;
@@ -443,12 +288,6 @@ int launch_buf_t(const BufMergeArgs& a, cudaStream_t s) {
 }
 
 }  // namespace
-
-int launch_ctx_attn_simt(const CtxAttnArgs& a, cudaStream_t s) {
-  if (a.rows <= 0) return ARTAB_OK;
-  ARTAB_REQUIRE(a.n_ctx > 0 && a.n_splits >= 1, ARTAB_EINVAL, "context attention: empty context or no splits");
-  return a.dtype == ARTAB_BF16 ? launch_ctx_t<__nv_bfloat16>(a, s) : launch_ctx_t<float>(a, s);
-}
 
 int launch_buf_merge(const BufMergeArgs& a, cudaStream_t s) {
   if (a.n_items <= 0) return ARTAB_OK;

@@ -55,6 +55,7 @@ struct DenseArgs {
   int pair_slots;      // slots in pair_scratch; a pair uses 6: MLP exchange (0, 1), head exchange (2, 3), parking (4, 5)
   const void *tc_wa, *tc_wb;  // tensor-core tiles of the head matrices (null: fp32 chain)
   int tc_head_lo;
+  const float* fma_head;      // D x D panels of the head, see artab_model
 #ifdef ARTAB_TIMELINE
   int tl_slot;         // diagnostic builds: which timeline slot this launch stamps
 #endif
@@ -63,6 +64,8 @@ struct DenseArgs {
 int launch_embed(const EmbedArgs& a, cudaStream_t s);
 int launch_dense(const DenseArgs& a, cudaStream_t s);     // picks the tensor-core chain when it applies
 int launch_dense_tc(const DenseArgs& a, cudaStream_t s);  // tcgen05 chain (bf16 mode)
+int launch_dense_fma(const DenseArgs& a, cudaStream_t s); // register-tiled fp32 chain (d_model 64, 128, 192)
+bool dense_fma_applicable(const DenseArgs& a);
 bool dense_tc_applicable(const DenseArgs& a);
 bool chain_on_tc(const artab_model* m, const artab_state* st);  // every dense launch of this model takes the tcgen05 chain
 

@@ -89,6 +89,11 @@ typedef struct artab_layer_weights {
   const void* tc_wqkv;
   int32_t tc_lo;        /* bit 0 wo, 1 w1, 2 w2, 3 wf, 4 wqkv: the matrix carries lo slabs */
   int32_t tc_reserved;
+  /* Optional fp32 copies in D x D panels ([in][out] inside a panel), one after the other in the order of use
+   * (d_model 64, 128, 192 and d_ff a multiple of it; NULL: the 8-row kernel runs):
+   *   fma_pre: wf, q, k, v;  fma_post: wo, then per D-wide chunk j of the hidden layer w1[:, j], w2[j, :]. */
+  const float* fma_pre;
+  const float* fma_post;
 } artab_layer_weights;
 
 typedef struct artab_model {
@@ -113,6 +118,7 @@ typedef struct artab_model {
   int32_t tc_head_lo;        /* bit 0 wa, bit 1 wb */
   int32_t tc_reserved;
   const artab_layer_weights* layers; /* HOST pointer to n_layers entries */
+  const float* fma_head;             /* per D-wide chunk j: wa[:, j], then wb[j, :] padded to D columns (or NULL) */
   /* whole-sequence decode (NULL: artab_decode_sequence is not available): per cluster rank one contiguous
    * stream of the matrix slices that rank uses, in the order of use, fp32 in units of 32 k x 16 columns (_pack.py);
    * seq_ranks is the largest divisor of n_heads that is at most 8 */
