@@ -30,6 +30,12 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool vali
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(n) : "memory");
 }
 
+// four neighbouring elements from an address that only has the element's alignment
+template <typename T>
+__device__ __noinline__ float4 load4_any(const T* p) {
+  return make_float4(to_f32<T>(p[0]), to_f32<T>(p[1]), to_f32<T>(p[2]), to_f32<T>(p[3]));
+}
+
 template <typename T, int DH, int NR>
 __global__ void __launch_bounds__(kWarps * 32, 2) ctx_attn_fma_kernel(const CtxAttnArgs a) {
   extern __shared__ __align__(128) uint8_t raw[];
@@ -52,6 +58,10 @@ __global__ void __launch_bounds__(kWarps * 32, 2) ctx_attn_fma_kernel(const CtxA
   const T* Kc = reinterpret_cast<const T*>(a.k_ctx) + (size_t)(g * a.n_heads + h) * a.n_ctx_pad * DH;
   const T* Vc = reinterpret_cast<const T*>(a.v_ctx) + (size_t)(g * a.n_heads + h) * a.n_ctx_pad * DH * (a.v_transposed ? 2 : 1);
 
+  // A caller's own K / V may start anywhere, and transposed V may have any pitch: wide loads need 16-byte aligned
+  // arrays and pitches of whole float4s.
+  const bool wide = (((uintptr_t)a.k_ctx | (uintptr_t)a.v_ctx) & 15) == 0 && (!a.v_transposed || (a.n_ctx_pad & 3) == 0);
+
   // keys [k0, k0 + 64) -> stage st; float4 (key, dims 4d .. 4d + 3) of K sits at [d / 4][key % 4][d % 4][key / 4], of V at
   // [key % NI][key / NI][d]
   auto stage = [&](int k0, int st) {
@@ -61,11 +71,14 @@ __global__ void __launch_bounds__(kWarps * 32, 2) ctx_attn_fma_kernel(const CtxA
       float4* vd = &sm.kv[st][t][8 * DH + (kt & (NI - 1)) * 32 + kt / NI * D4 + d];
       const bool valid = k0 + key < k_end;
       const size_t at = (size_t)(valid ? k0 + key : 0) * DH + 4 * d;
-      if constexpr (sizeof(T) == 4) {
+      const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (!wide) {
+        *kd = valid ? load4_any(Kc + at) : z;
+        if (!a.v_transposed) *vd = valid ? load4_any(Vc + at) : z;
+      } else if constexpr (sizeof(T) == 4) {
         cp_async16(kd, Kc + at, valid);
-        cp_async16(vd, Vc + at, valid);
+        if (!a.v_transposed) cp_async16(vd, Vc + at, valid);
       } else {
-        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
         *kd = valid ? load4(Kc + at) : z;
         if (!a.v_transposed) *vd = valid ? load4(Vc + at) : z;
       }
@@ -75,8 +88,13 @@ __global__ void __launch_bounds__(kWarps * 32, 2) ctx_attn_fma_kernel(const CtxA
         for (int i = tid; i < DH * (kStage / 4); i += kWarps * 32) {
           const int d = i / (kStage / 4), key = 4 * (i - d * (kStage / 4)), t = key >> 5, kt = key & 31;
           float v[4] = {0.f, 0.f, 0.f, 0.f};
-          if (k0 + key < k_end) {   // the cache is padded to a multiple of eight keys
-            const float4 hi = load4(Vc + (size_t)d * a.n_ctx_pad + k0 + key), lo = load4(Vc + (size_t)(DH + d) * a.n_ctx_pad + k0 + key);
+          const T* vp = Vc + (size_t)d * a.n_ctx_pad + k0 + key;
+          if (!wide) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (k0 + key + e < k_end) v[e] = to_f32<T>(vp[e]) + to_f32<T>(vp[(size_t)DH * a.n_ctx_pad + e]);
+          } else if (k0 + key < k_end) {   // a pitch of whole float4s: the last one may reach into the padding
+            const float4 hi = load4(vp), lo = load4(vp + (size_t)DH * a.n_ctx_pad);
             v[0] = hi.x + lo.x; v[1] = hi.y + lo.y; v[2] = hi.z + lo.z; v[3] = hi.w + lo.w;
           }
 #pragma unroll
@@ -129,7 +147,12 @@ __global__ void __launch_bounds__(kWarps * 32, 2) ctx_attn_fma_kernel(const CtxA
     const float4 o = *reinterpret_cast<const float4*>(&sm.pw[warp][r * DH + d]);
     const size_t ro = ((size_t)split * a.rows + row) * a.n_heads + h;
     float* dst = a.out + (a.out_lane_major ? lane_major_index(row, h * DH + d, a.n_heads * DH) : ro * DH + d);
-    *reinterpret_cast<float4*>(dst) = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
+    const float4 y = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
+    if (((uintptr_t)a.out & 15) == 0) {
+      *reinterpret_cast<float4*>(dst) = y;
+    } else {
+      dst[0] = y.x; dst[1] = y.y; dst[2] = y.z; dst[3] = y.w;
+    }
     if (d == 0) a.lse[ro] = l > 0.f ? (m + log2f(l)) * kLn2 : -INFINITY;
   }
 }
@@ -180,8 +203,6 @@ int launch_ctx_attn_simt(const CtxAttnArgs& a, cudaStream_t s) {
   ARTAB_REQUIRE(a.n_ctx > 0 && a.n_splits >= 1, ARTAB_EINVAL, "context attention: empty context or no splits");
   ARTAB_REQUIRE(a.head_dim == 16 || a.head_dim == 32 || a.head_dim == 64, ARTAB_EINVAL,
                 "context attention: head_dim %d not supported (16, 32, 64)", a.head_dim);
-  ARTAB_REQUIRE(((uintptr_t)a.k_ctx % 16) == 0 && ((uintptr_t)a.v_ctx % 16) == 0, ARTAB_EINVAL,
-                "context attention: k / v must be 16-byte aligned");
   return a.dtype == ARTAB_BF16 ? launch_t<__nv_bfloat16>(a, s) : launch_t<float>(a, s);
 }
 

@@ -45,3 +45,49 @@ def test_fp32_joint_density_at_tile_edges(case):
     noise = float((want.double() - want64).pow(2).mean().sqrt())
     err = (got - want).abs()
     assert bool((err <= 1e-5 * (1 + want.abs()) + 4 * noise).all()), (float(err.max()), noise)
+
+
+# dtype, head size, keys, pitch of the key axis, elements K / V / out start after a 16-byte boundary
+PLACES = [
+    (torch.bfloat16, 16, 50, 50, 0),    # transposed V with a pitch of no whole float4s
+    (torch.bfloat16, 64, 70, 71, 0),    # odd pitch
+    (torch.bfloat16, 16, 33, 40, 3),    # whole pitch, arrays off the boundary
+    (torch.float32, 32, 65, 65, 1),
+    (torch.float32, 64, 40, 41, 2),
+]
+
+
+@pytest.mark.parametrize("place", PLACES, ids=lambda p: "%s_dh%d_nc%d_pitch%d_off%d" % (str(p[0])[6:], *p[1:]))
+def test_context_attention_takes_any_placement(place):
+    import ar_tabpfn  # noqa: F401
+    from ar_tabpfn import _lib
+    dtype, Dh, Nc, Ncp, off = place
+    H, rows = 2, 11
+    g = torch.Generator().manual_seed(Nc)
+    q, k, v = (torch.randn(n, H, Dh, generator=g).to(dtype) for n in (rows, Nc, Nc))
+    kp = torch.zeros(H, Ncp, Dh, dtype=dtype)
+    kp[:, :Nc] = k.transpose(0, 1)
+    if dtype == torch.bfloat16:
+        vp = torch.zeros(H, 2 * Dh, Ncp, dtype=dtype)
+        vp[:, :Dh, :Nc] = v.permute(1, 2, 0)
+    else:
+        vp = torch.zeros(H, Ncp, Dh, dtype=dtype)
+        vp[:, :Nc] = v.transpose(0, 1)
+
+    def placed(t):
+        buf = torch.zeros(t.numel() + off + 8, dtype=t.dtype, device="cuda")
+        at = buf[off:off + t.numel()]
+        at.copy_(t.reshape(-1))
+        return at
+
+    kd, vd, out = placed(kp), placed(vp), placed(torch.zeros(rows, H, Dh))
+    qd, lse = q.cuda(), torch.empty(rows, H, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    _lib.check(_lib.lib().artab_context_attention(_lib.dtype_code(dtype), _lib.ptr(qd), _lib.ptr(kd), _lib.ptr(vd), rows,
+                                                  rows, 1, H, Dh, Nc, Ncp, 1, _lib.ptr(out), _lib.ptr(lse),
+                                                  _lib.ptr(status), _lib.stream_ptr()))
+    s = torch.einsum("rhd,khd->rhk", q.double(), k.double()) / Dh ** 0.5
+    want = torch.einsum("rhk,khd->rhd", s.softmax(-1), v.double())
+    # fp32 arithmetic on the stored values: sums over at most 70 keys
+    torch.testing.assert_close(out.view(rows, H, Dh).cpu().double(), want, atol=1e-5, rtol=1e-5)
+    torch.testing.assert_close(lse.cpu().double(), s.logsumexp(-1), atol=1e-5, rtol=1e-5)
