@@ -24,7 +24,8 @@ _fp = C.c_void_p  # every device pointer travels as void*
 class LayerWeights(C.Structure):
     _fields_ = [(n, _fp) for n in ("wf_t", "ln1_g", "ln1_b", "wqkv_t", "wo_t", "ln2_g", "ln2_b", "w1_t", "b1",
                                    "w2_t", "b2", "ln3_g", "ln3_b", "tc_wo", "tc_w1", "tc_w2", "tc_wf", "tc_wqkv")] + \
-               [("tc_lo", C.c_int32), ("tc_reserved", C.c_int32), ("fma_pre", _fp), ("fma_post", _fp)]
+               [("tc_lo", C.c_int32), ("tc_reserved", C.c_int32), ("fma_pre", _fp), ("fma_post", _fp),
+                ("mma_pre", _fp), ("mma_post", _fp)]
 
 
 class Model(C.Structure):
@@ -34,7 +35,7 @@ class Model(C.Structure):
                                    "wb_t", "bb", "mean_bias", "std_bias", "weight_bias", "tc_wa", "tc_wb")] + \
                [("tc_head_lo", C.c_int32), ("tc_reserved", C.c_int32), ("layers", C.POINTER(LayerWeights)),
                 ("fma_head", _fp), ("seq_w", _fp), ("seq_rank_bytes", C.c_int64), ("seq_vec_off", C.c_int64),
-                ("seq_ranks", C.c_int32), ("seq_reserved", C.c_int32)]
+                ("seq_ranks", C.c_int32), ("seq_reserved", C.c_int32), ("mma_head", _fp)]
 
 
 class State(C.Structure):

@@ -129,7 +129,7 @@ class PackedModel:
         self._layers = (_lib.LayerWeights * self.n_layers)()
         for i in range(self.n_layers):
             for f, _ in _lib.LayerWeights._fields_:
-                if not f.startswith(("tc_", "fma_")):
+                if not f.startswith(("tc_", "fma_", "mma_")):
                     setattr(self._layers[i], f, P(f"{i}.{f}"))
         m = _lib.Model()
         m.d_model, m.n_heads, m.head_dim, m.d_ff = self.d_model, self.n_heads, self.head_dim, self.d_ff
@@ -142,6 +142,7 @@ class PackedModel:
         self._pack_tensor_core(embedder, backbone, head, target)
         self._pack_sequence(dict(items), target)
         self._pack_panels(dict(items), target)
+        self._pack_fragments(dict(items), target)
 
     def _pack_tensor_core(self, embedder, backbone, head, target):
         """bf16 hi/lo tiles for the tcgen05 per-token chain (d_model in {64,128,192}, d_ff % 128 == 0,
@@ -269,6 +270,42 @@ class PackedModel:
             else:
                 setattr(self._layers[n // 2], ("fma_pre", "fma_post")[n % 2], at)
             at += 4 * D * D * len(st)
+
+    def _pack_fragments(self, w, target):
+        """mma.m16n8k16 B fragments for the few-row bf16 chain: four slices of every matrix (by output column, w2 and
+        head.2 by input row), hi part then lo part.  A part is a sequence of units of 8 columns x 32 k, k innermost;
+        in a unit lane (g, t) holds column g, k = 16 ks + 8 half + 2 t + e at [ks][half][e]."""
+        self.mma_flat = None
+        if self.tc_flat is None:
+            return
+        D, Dff, K = self.d_model, self.d_ff, self.n_comp
+        ds, hs = D // 4, Dff // 4
+        wb = torch.zeros(Dff, 16, dtype=torch.float64)
+        wb[:, :3 * K] = w["wb_t"]
+
+        def parts(m):
+            u = lambda t: t.reshape(m.shape[0] // 32, 2, 2, 4, 2, m.shape[1] // 8, 8).permute(5, 0, 6, 3, 1, 2, 4).reshape(-1)
+            hi, lo = _split_bf16(m)
+            return [u(hi.to(torch.bfloat16)), u(lo.to(torch.bfloat16))]
+
+        def streams(matrices):
+            return torch.cat([p for r in range(4) for m in matrices(r) for p in parts(m.contiguous())])
+
+        cols = lambda m, r: m[:, r * m.shape[1] // 4:(r + 1) * m.shape[1] // 4]
+        rows = lambda m, r: m[r * hs:(r + 1) * hs]
+        stacks = []
+        for i in range(self.n_layers):
+            stacks.append(streams(lambda r: [cols(w[f"{i}.wf_t"], r), torch.cat([cols(m, r) for m in w[f"{i}.wqkv_t"].split(D, dim=1)], dim=1)]))
+            stacks.append(streams(lambda r: [cols(w[f"{i}.wo_t"], r), cols(w[f"{i}.w1_t"], r), rows(w[f"{i}.w2_t"], r)]))
+        stacks.append(streams(lambda r: [cols(w["wa_t"], r), rows(wb, r)]))
+        self.mma_flat = torch.cat(stacks).to(target)
+        at = self.mma_flat.data_ptr()
+        for n, st in enumerate(stacks):
+            if n == len(stacks) - 1:
+                self.struct.mma_head = at
+            else:
+                setattr(self._layers[n // 2], ("mma_pre", "mma_post")[n % 2], at)
+            at += 2 * st.numel()
 
     @property
     def ref(self):

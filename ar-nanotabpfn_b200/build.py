@@ -17,7 +17,7 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libartab_b200.so")
 # (source, object name, extra defines)
 SOURCES = [(f, f[:-3], []) for f in ("api.cu", "dense_simt.cu", "attn_simt.cu", "attn_fma.cu", "attn_tc.cu", "buf_mma.cu", "noalloc.cu",
-                                     "dense_tc.cu", "dense_fma.cu", "seq.cu")]
+                                     "dense_tc.cu", "dense_fma.cu", "dense_mma.cu", "seq.cu")]
 # the whole-sequence kernel has many variants: one compiler process per cache type and head size
 SOURCES += [("seq_simt.cu", f"seq_simt_{'bf16' if b else 'f32'}_{dh}", [f"-DARTAB_SEQ_BF16={b}", f"-DARTAB_SEQ_DH={dh}"])
             for b in (0, 1) for dh in (16, 32, 64)]

@@ -222,6 +222,7 @@ void fill_head(const artab_model* m, DenseArgs& d) {
   d.tc_wb = m->tc_wb;
   d.tc_head_lo = m->tc_head_lo;
   d.fma_head = m->fma_head;
+  d.mma_head = m->mma_head;
 }
 
 DenseArgs dense_base(const artab_model* m, const artab_state* st, int rows) {

@@ -56,6 +56,7 @@ struct DenseArgs {
   const void *tc_wa, *tc_wb;  // tensor-core tiles of the head matrices (null: fp32 chain)
   int tc_head_lo;
   const float* fma_head;      // D x D panels of the head, see artab_model
+  const void* mma_head;       // the head in fragment order, see artab_model
 #ifdef ARTAB_TIMELINE
   int tl_slot;         // diagnostic builds: which timeline slot this launch stamps
 #endif
@@ -65,6 +66,8 @@ int launch_embed(const EmbedArgs& a, cudaStream_t s);
 int launch_dense(const DenseArgs& a, cudaStream_t s);     // picks the tensor-core chain when it applies
 int launch_dense_tc(const DenseArgs& a, cudaStream_t s);  // tcgen05 chain (bf16 mode)
 int launch_dense_fma(const DenseArgs& a, cudaStream_t s); // register-tiled fp32 chain (d_model 64, 128, 192)
+int launch_dense_mma(const DenseArgs& a, cudaStream_t s); // bf16 chain for few rows (clusters of four CTAs)
+bool dense_mma_applicable(const DenseArgs& a);
 bool dense_fma_applicable(const DenseArgs& a);
 bool dense_tc_applicable(const DenseArgs& a);
 bool chain_on_tc(const artab_model* m, const artab_state* st);  // every dense launch of this model takes the tcgen05 chain

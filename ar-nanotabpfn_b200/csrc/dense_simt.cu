@@ -475,6 +475,7 @@ int launch_embed(const EmbedArgs& a, cudaStream_t s) {
 
 int launch_dense(const DenseArgs& a, cudaStream_t s) {
   if (a.rows <= 0) return ARTAB_OK;
+  if (dense_mma_applicable(a)) return launch_dense_mma(a, s);
   if (dense_tc_applicable(a)) return launch_dense_tc(a, s);
   if (dense_fma_applicable(a)) return launch_dense_fma(a, s);
   ARTAB_REQUIRE(a.D % 32 == 0 && a.Dff % 4 == 0 && a.D >= 32, ARTAB_EINVAL,

@@ -94,6 +94,11 @@ typedef struct artab_layer_weights {
    *   fma_pre: wf, q, k, v;  fma_post: wo, then per D-wide chunk j of the hidden layer w1[:, j], w2[j, :]. */
   const float* fma_pre;
   const float* fma_post;
+  /* Optional bf16 copies in mma.m16n8k16 fragment order for the few-row chain (NULL: the tcgen05 chain runs): four
+   * slices by output column (w2: by input row), each the hi part and the lo part of every matrix one after the other:
+   *   mma_pre: wf, q | k | v;  mma_post: wo, w1, w2 (_pack.py). */
+  const void* mma_pre;
+  const void* mma_post;
 } artab_layer_weights;
 
 typedef struct artab_model {
@@ -126,6 +131,7 @@ typedef struct artab_model {
   int64_t seq_rank_bytes, seq_vec_off;  /* bytes per rank; where its LayerNorm and bias vectors start */
   int32_t seq_ranks;
   int32_t seq_reserved;
+  const void* mma_head;                 /* head.head.0, head.head.2 padded to 16 columns, as mma_post (or NULL) */
 } artab_model;
 
 /* ------------------------------------------------------------------------- */
