@@ -1,6 +1,7 @@
 // Host side of the whole-sequence decode: applicability, shared-memory plan, context re-tiling, launch.
 #include <cstring>
 
+#include "attn.cuh"
 #include "dense.cuh"
 #include "seq.cuh"
 
@@ -11,6 +12,7 @@ namespace {
 constexpr size_t kSmemMax = 227 * 1024;
 constexpr long long kWaitCycles = 2000000000LL;  // about one second
 constexpr int kMaxRowsPerCluster = 16;
+constexpr size_t kWorkspaceMax = (size_t)4 << 30;
 
 inline int largest_divisor(int n, int most) {
   for (int c = most; c > 1; --c)
@@ -99,10 +101,6 @@ bool seq_plan(const artab_model* m, const artab_state* st, SeqPlan& p, SeqArgs& 
   if (C != m->seq_ranks || !(D == 64 || D == 128 || D == 192) || !(DH == 16 || DH == 32 || DH == 64)) return false;
   const int DS = D / C, HS = m->d_ff / C, NB = (3 * m->n_comp + 15) & ~15;
   if (D % C || m->d_ff % C || DS % 16 || HS % 32 || HS > 192 || 3 * DS > 192) return false;
-  // Where the launch-per-layer path runs on tensor cores its time hardly depends on the number of streams
-  // (270 us per target up to 512 of them), while this kernel's grows with the streams per cluster: 120 us at 32
-  // streams, 240 us at 64 with a context each.
-  if (chain_on_tc(m, st) && st->n_streams > 64) return false;
   // streams per cluster: as few as one wave of clusters needs, at most what the variants hold
   const int most = kMaxRowsPerCluster / 2;
   static thread_local int clusters[9][kMaxDevices];
@@ -111,8 +109,23 @@ bool seq_plan(const artab_model* m, const artab_state* st, SeqPlan& p, SeqArgs& 
   int& fit = clusters[C][dev];
   if (!fit) fit = seq_simt_max_clusters(C, kSmemMax);
   if (fit <= 0) return false;
-  const int waves = (st->n_streams + fit * most - 1) / (fit * most);
-  const int spc = (st->n_streams + waves * fit - 1) / (waves * fit);
+  // One wave: a second one doubles the time, while the launch-per-layer path hardly notices (fp32, 512 context
+  // rows, 8 targets, d_model 128, 6 layers: 2.3 against 3.4 ms at 128 streams, 4.9 against 3.7 at 512, 16.5 against
+  // 6.6 at 2048).
+  if (st->n_streams > fit * most) return false;
+  // the re-tiled copy of the context is as large as its fp32 cache: not where that is a good part of the memory
+  if (context_bytes(m, st) > kWorkspaceMax) return false;
+  const int spc = (st->n_streams + fit - 1) / fit;
+  // Models whose launch-per-layer path runs on tensor cores.  That path hardly notices the number of streams, this
+  // kernel walks up to four rows per cluster at the same speed and more at a lower one (6 layers, d_model 192, 1000
+  // context rows, 8 targets: 1.9 against 2.3 ms at 32 streams, 2.7 against 2.3 at 48); nor does that path notice
+  // the context as much where the contraction is on tensor cores too (24 streams: 2.3 against 2.5 ms at 2000 rows,
+  // 3.0 against 2.7 at 4000).  A context per stream leaves its 128-query tiles nearly empty: 3.5 against 3.9 ms for
+  // 64 datasets of 500 rows, equal at 96.
+  if (chain_on_tc(m, st)) {
+    if (st->n_groups > 1 ? st->n_streams > 64 : spc > 2) return false;
+    if (st->n_groups == 1 && ctx_attn_tc_supported(st->dtype, DH) && st->n_ctx > 3000) return false;
+  }
   const int R = spc <= 1 ? 2 : spc <= 2 ? 4 : spc <= 4 ? 8 : kMaxRowsPerCluster;
   const Areas ar = areas_of(m, C, R);
   const size_t fixed = kSeqBarBytes + 4 * ((size_t)ar.red + ar.area);
