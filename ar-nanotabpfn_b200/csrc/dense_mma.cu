@@ -12,7 +12,9 @@
 //
 // What bounds it: a chain of about twelve short phases; a product phase is bounded by the shared-memory reads of the
 // activation operand (each warp reads all 32 rows for its 16 columns).  512 streams x 128 targets on 1024 context rows,
-// 6 layers, d_model 192: 44.8 ms per sampling job with the tcgen05 chain, 32.9 ms with this one.
+// 6 layers, d_model 192: 44.8 ms per sampling job with the tcgen05 chain, 32.4 ms with this one (40 K cycles from the
+// end of the wait to the last store).  One rolled loop for all products, so that their instructions are fetched once,
+// was slower (37.1 ms).
 #include "cluster.cuh"
 #include "dense.cuh"
 #include "head.cuh"
@@ -83,7 +85,7 @@ __device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t addr) {
                : "memory");
 }
 __device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
@@ -125,23 +127,28 @@ struct Frags {
 // acc[m tile][n tile] += act . w over n blocks of 32 k; PARTS 2: hi and lo part of the activations, 1: the hi part
 template <int PARTS, int NU>
 __device__ __forceinline__ void multiply(float (&acc)[2][2][4], const Frags<NU>& f, const Operand& x, int u0, int n) {
+  // the fragments of a k step are read while the MMAs of the step before it run
+  uint32_t a[2][2][PARTS][4];
+  auto read = [&](int step) {
 #pragma unroll
-  for (int u = 0; u < NU; ++u) {
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int part = 0; part < PARTS; ++part)
+        ldmatrix4(a[step & 1][m][part], x.base + part * x.lo + m * 16 * x.pitch + u0 * 64 + step * 32);
+  };
+  read(0);
+#pragma unroll
+  for (int step = 0; step < 2 * NU; ++step) {
+    const int u = step >> 1;
     if (u < n) {
+      if (step + 1 < 2 * NU && (step + 1) >> 1 < n) read(step + 1);
 #pragma unroll
-      for (int ks = 0; ks < 2; ++ks) {
+      for (int part = 0; part < PARTS; ++part)
 #pragma unroll
-        for (int m = 0; m < 2; ++m) {
+        for (int m = 0; m < 2; ++m)
 #pragma unroll
-          for (int part = 0; part < PARTS; ++part) {
-            uint32_t a[4];
-            ldmatrix4(a, x.base + part * x.lo + m * 16 * x.pitch + ((u0 + u) * 32 + ks * 16) * 2);
-#pragma unroll
-            for (int t = 0; t < 2; ++t)
-              mma(acc[m][t], a, ks ? f.w[t][u].z : f.w[t][u].x, ks ? f.w[t][u].w : f.w[t][u].y);
-          }
-        }
-      }
+          for (int t = 0; t < 2; ++t)
+            mma(acc[m][t], a[step & 1][m][part], step & 1 ? f.w[t][u].z : f.w[t][u].x, step & 1 ? f.w[t][u].w : f.w[t][u].y);
     }
   }
 }
@@ -179,7 +186,7 @@ __device__ __forceinline__ void store_split(uint8_t* operand, int k, int row, in
 // act <- LayerNorm(res + xg + bias) as hi and lo part; res <- the same unless it is the last use; optional copy of this
 // CTA's eight rows to global memory.  Eight lanes per row.  `x`: the exchange that brings xg (-1: none).
 template <int D>
-__device__ __noinline__ void layer_norm(float* res, const float* xg, const float* bias, const float* gamma, const float* beta,
+__device__ __forceinline__ void layer_norm(float* res, const float* xg, const float* bias, const float* gamma, const float* beta,
                                         uint8_t* act, int x, float* copy, int rank, int n_valid) {
   constexpr int N = D / 32, P = D + 4;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -276,22 +283,16 @@ __global__ void __launch_bounds__(kThreads, 1) dense_mma_kernel(const __grid_con
   float* v_ln2g = vec, *v_ln2b = vec + D, *v_b2 = vec + 2 * D, *v_ln3g = vec + 3 * D, *v_ln3b = vec + 4 * D;
   float* v_ln1g = vec + 5 * D, *v_ln1b = vec + 6 * D, *v_lnfg = vec + 7 * D, *v_lnfb = vec + 8 * D;
   float* v_b1 = vec + 9 * D, *v_ba = v_b1 + HS;
-  if (tid < D) {
-    if (a.do_post) {
-      v_ln2g[tid] = __ldg(a.post_w.ln2_g + tid);
-      v_ln2b[tid] = __ldg(a.post_w.ln2_b + tid);
-      v_b2[tid] = __ldg(a.post_w.b2 + tid);
-      v_ln3g[tid] = __ldg(a.post_w.ln3_g + tid);
-      v_ln3b[tid] = __ldg(a.post_w.ln3_b + tid);
-    }
-    if (a.do_pre) {
-      v_ln1g[tid] = __ldg(a.pre_w.ln1_g + tid);
-      v_ln1b[tid] = __ldg(a.pre_w.ln1_b + tid);
-    }
-    if (a.do_final) {
-      v_lnfg[tid] = __ldg(a.lnf_g + tid);
-      v_lnfb[tid] = __ldg(a.lnf_b + tid);
-    }
+  if (tid < D) {   // every load before the first store: one round trip
+    const bool post = a.do_post, pre = a.do_pre, fin = a.do_final;
+    const float* src[9] = {post ? a.post_w.ln2_g : nullptr, post ? a.post_w.ln2_b : nullptr, post ? a.post_w.b2 : nullptr,
+                           post ? a.post_w.ln3_g : nullptr, post ? a.post_w.ln3_b : nullptr, pre ? a.pre_w.ln1_g : nullptr,
+                           pre ? a.pre_w.ln1_b : nullptr,   fin ? a.lnf_g : nullptr,         fin ? a.lnf_b : nullptr};
+    float v[9];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) v[i] = src[i] ? __ldg(src[i] + tid) : 0.f;
+#pragma unroll
+    for (int i = 0; i < 9; ++i) vec[i * D + tid] = v[i];
   }
   for (int i = tid; i < HS; i += kThreads) {
     if (a.do_post) v_b1[i] = __ldg(a.post_w.b1 + rank * HS + i);
@@ -316,18 +317,26 @@ __global__ void __launch_bounds__(kThreads, 1) dense_mma_kernel(const __grid_con
 
   // ---- rows in ----
   {
-    const float4* src = reinterpret_cast<const float4*>(a.do_post ? a.attn : a.x_in);
+    const float4* src = reinterpret_cast<const float4*>(a.do_post ? a.attn : a.x_in) + row0 * (D / 4);
+    const float4* s1 = reinterpret_cast<const float4*>(a.do_post ? a.x1_in : a.x_in) + row0 * (D / 4);
     const bool lm = a.do_post || a.x_in_lane_major;
-    const float4* s1 = reinterpret_cast<const float4*>(a.x1_in) + row0 * (D / 4);
+    constexpr int NI = (kRows * D / 4 + kThreads - 1) / kThreads;
+    float4 v[NI], r[NI];
 #pragma unroll
-    for (int j = 0; j < kRows * D / 4 / kThreads + 1; ++j) {
+    for (int j = 0; j < NI; ++j) {
+      const int i = tid + j * kThreads;
+      const bool ok = i < kRows * D / 4 && (lm || i / (D / 4) < n_valid);
+      v[j] = ok ? src[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+      r[j] = ok ? s1[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int j = 0; j < NI; ++j) {
       const int i = tid + j * kThreads;
       if (i < kRows * D / 4) {
         const int row = lm ? i & 31 : i / (D / 4), c4 = lm ? i >> 5 : i - row * (D / 4);
-        const float4 v = lm || row < n_valid ? src[row0 * (D / 4) + i] : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float y[4] = {v.x, v.y, v.z, v.w};
+        const float y[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
         store_split(act, D, row, 4 * c4, y);
-        *reinterpret_cast<float4*>(res + row * P + 4 * c4) = a.do_post ? s1[i] : v;
+        *reinterpret_cast<float4*>(res + row * P + 4 * c4) = r[j];
       }
     }
   }
@@ -388,16 +397,22 @@ __global__ void __launch_bounds__(kThreads, 1) dense_mma_kernel(const __grid_con
     if (hid_active) wide.load(w1, warp, NU, 0, NU);
     layer_norm<D>(res, xa, nullptr, v_ln2g, v_ln2b, act, 0, nullptr, rank, n_valid);
     hidden(wide, w1, lo_post & 2, v_b1);
-    Frags<8> deep;
+    constexpr int ND = 6;   // blocks of 32 k held at once
+    Frags<ND> deep;
     const bool w2_active = warp < D / 16;
-    if (w2_active) deep.load(w2, warp, KU, 0, KU);
+    if (w2_active) deep.load(w2, warp, KU, 0, min(KU, ND));
     __syncthreads();
     if (w2_active) {
       zero(acc);
-      multiply<2>(acc, deep, x_hid, 0, KU);
-      if (lo_post & 4) {
-        deep.load(w2 + WH, warp, KU, 0, KU);
-        multiply<1>(acc, deep, x_hid, 0, KU);
+#pragma unroll 1
+      for (int u = 0; u < KU; u += ND) {
+        const int n = min(KU - u, ND);
+        if (u) deep.load(w2, warp, KU, u, n);
+        multiply<2>(acc, deep, x_hid, u, n);
+        if (lo_post & 4) {
+          deep.load(w2 + WH, warp, KU, u, n);
+          multiply<1>(acc, deep, x_hid, u, n);
+        }
       }
       const int owner = 16 * warp / DS;
       const uint32_t at = map_to_rank(smem_u32(part + rank * kRows * DS + 16 * warp - owner * DS), owner);
@@ -469,6 +484,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_mma_kernel(const __grid_con
     const bool qkv_active = warp < 3 * PAIRS;
     if (qkv_active) wide.load(wq, warp, NU, 0, NU);
     layer_norm<D>(res, xa, nullptr, v_ln1g, v_ln1b, act, 3, a.x1_out + row0 * D, rank, n_valid);
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // nobody sends any more
     if (qkv_active) {
       zero(acc);
       multiply<2>(acc, wide, x_act, 0, NU);
@@ -488,15 +504,16 @@ __global__ void __launch_bounds__(kThreads, 1) dense_mma_kernel(const __grid_con
       }
     }
   }
-  // nobody leaves while a peer could still write here (after a wait that gave up, stores may be in flight)
+  // nobody leaves while a peer could still write here
+  __syncthreads();
+  if (a.do_head) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (bars->abort_flag) {
     if (tid == 0 && a.status) atomicExch(a.status, 6);
     const long long t0 = clock64();
-    while (clock64() - t0 < 100000) {
+    while (clock64() - t0 < 100000) {   // after a wait that gave up, a peer's stores may be in flight
     }
   }
-  __syncthreads();
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // rows of the clusters that fit the GPU at once
@@ -545,7 +562,7 @@ int launch_d(const DenseArgs& a, cudaStream_t s) {
 
 // One wave of clusters: beyond it the tcgen05 chain, whose time hardly grows up to 148 row tiles, is the faster one.
 bool dense_mma_applicable(const DenseArgs& a) {
-  if (!a.lane_major || a.x_out || a.z_out || !dense_tc_applicable(a)) return false;
+  if (!a.lane_major || !(a.do_pre || (a.do_post && a.do_head)) || a.x_out || a.z_out || !dense_tc_applicable(a)) return false;
   if ((a.do_post && !a.post_w.mma_post) || (a.do_pre && !a.pre_w.mma_pre) || (a.do_head && !a.mma_head)) return false;
   const size_t smem = plan_of(a.D, a.Dff / kC).total;
   const int most = a.D == 64 ? rows_at_once<64>(smem) : a.D == 128 ? rows_at_once<128>(smem) : rows_at_once<192>(smem);
