@@ -22,6 +22,9 @@ from .. import _lib
 from .._pack import packed_for
 
 
+_CACHE_VIEWS = ("k_ctx_cache", "v_ctx_cache", "k_buf_cache", "v_buf_cache")
+
+
 def _pad8(n: int) -> int:
     return (n + 7) // 8 * 8
 
@@ -60,6 +63,8 @@ class ARTabPFNPredictor:
         self._max_seq = 0
         self._state: Optional[_lib.State] = None
         self._bufs = {}
+        self._laid_out = None
+        self._views = []
         self.last_logdens: Optional[Tensor] = None
         self.last_components: Optional[Tensor] = None
         self.last_h2d_bytes = 0
@@ -147,9 +152,9 @@ class ARTabPFNPredictor:
             self._bufs[name] = t
         return t[:n].view(*shape)
 
-    def _ensure_rows(self, rows: int) -> None:
+    def _ensure_rows(self, rows: int, pm) -> None:
         """Row workspaces (residual stream, queries, attention output, partials)."""
-        st, pm = self._state, self._packed(self._device)
+        st = self._state
         if rows <= st.max_rows:
             return
         D, H, Dh = pm.d_model, pm.n_heads, pm.head_dim
@@ -164,11 +169,10 @@ class ARTabPFNPredictor:
         st.max_rows = rows
         st.max_splits = _lib.MAX_SPLITS
 
-    def _layout(self, n_ctx: int) -> None:
+    def _layout(self, n_ctx: int, pm) -> None:
         """Allocate the layout-fixed caches: context K [L,G,H,Ncp,Dh], context V
         (in bf16 transposed and split hi | lo: [L,G,H,2Dh,Ncp]; the exposed
         ``v_ctx_cache`` view is the hi part) and the private buffers [L,B,H,T,2,Dh]."""
-        pm = self._packed(self._device)
         cdt = self._cache_dtype(self._dtype)
         B = self._batch
         G = 1 if self.shared else B
@@ -184,16 +188,25 @@ class ARTabPFNPredictor:
             v_ctx = self._alloc("v_ctx", (L, G, H, 2 * Dh, Ncp), cdt)  # hi | lo parts
         else:
             v_ctx = self._alloc("v_ctx", (L, G, H, Ncp, Dh), cdt)
-        k_ctx.zero_()
-        v_ctx.zero_()
         kv = self._alloc("kv_buf", (L, B, H, T, 2, Dh), cdt)
         st.k_ctx, st.v_ctx = k_ctx.data_ptr(), v_ctx.data_ptr()
         st.kv_buf = kv.data_ptr() if T > 0 else None
         st.status = self._alloc("status", (1,), torch.int32).data_ptr()
         self._state = st
         self.max_buffer_len = T
+        # The padding of the key axis is zero and nothing writes it: it is cleared when the layout changes.
+        layout = (k_ctx.data_ptr(), v_ctx.data_ptr(), kv.data_ptr(), cdt, L, B, G, H, T, Dh, n_ctx)
+        layers = list(self.backbone.layers)
+        if layout == self._laid_out and all(layer.__dict__.get(n) is t for layer, views in zip(layers, self._views)
+                                            for n, t in zip(_CACHE_VIEWS, views)):
+            return
+        if layout != self._laid_out:
+            k_ctx.zero_()
+            v_ctx.zero_()
+        self._laid_out = layout
+        self._views = []
         # reference-shaped views on the layer modules (inference.py:113-118)
-        for l, layer in enumerate(self.backbone.layers):
+        for l, layer in enumerate(layers):
             kc = k_ctx[l, :, :, :n_ctx]
             vc = (v_ctx[l, :, :, :Dh].transpose(-1, -2)[:, :, :n_ctx] if cdt == torch.bfloat16
                   else v_ctx[l, :, :, :n_ctx])
@@ -201,6 +214,7 @@ class ARTabPFNPredictor:
             layer.v_ctx_cache = vc[0] if self.shared else vc
             layer.k_buf_cache = kv[l, :, :, :, 0]
             layer.v_buf_cache = kv[l, :, :, :, 1]
+            self._views.append(tuple(getattr(layer, n) for n in _CACHE_VIEWS))
 
     # ---------------------------------------------------------------- status
     def _mirror_status(self) -> None:
@@ -241,9 +255,15 @@ class ARTabPFNPredictor:
     def prefill_context(self, x_context: Tensor, y_context: Tensor) -> None:
         """Encode the context rows and fill the context K/V of every layer.
         x_context [B,Nc,F], y_context [B,Nc]."""
-        lib = _lib.lib()
+        _lib.lib()
         if self._device is None:
             raise RuntimeError("init_kv_cache must be called before prefill_context")
+        self._prefill(x_context, y_context, self._packed(self._device))
+
+    def _prefill(self, x_context: Tensor, y_context: Tensor, pm) -> None:
+        """``pm``: the packed weights.  Looking every parameter over for changes is the larger part of the host
+        time of a small call: a whole-path call does it once and hands the result down."""
+        lib = _lib.lib()
         if x_context.is_cuda and x_context.device != self._device:
             raise ValueError("inputs must live on the cache device (or in host memory)")
         if self.shared:
@@ -253,11 +273,10 @@ class ARTabPFNPredictor:
         elif x_context.shape[0] != self._batch:
             raise ValueError("batch size differs from init_kv_cache")
         G, Nc, F = x_context.shape
-        self._layout(Nc)
-        self._ensure_rows(max(G * Nc, 2 * self._batch))
+        self._layout(Nc, pm)
+        self._ensure_rows(max(G * Nc, 2 * self._batch), pm)
         xc = self._dev32(x_context, self._device)
         yc = self._dev32(y_context, self._device).reshape(G, Nc)
-        pm = self._packed(self._device)
         _lib.check(lib.artab_prefill(pm.ref, C.byref(self._state), _lib.ptr(xc), _lib.ptr(yc), F,
                                      _lib.stream_ptr()))
         self.context_len = Nc
@@ -281,10 +300,10 @@ class ARTabPFNPredictor:
             raise RuntimeError("prefill_context must be called before decoding")
         if self.buffer_len + commit > self.max_buffer_len:
             raise ValueError("Shared-context buffer cache exceeded; increase max buffer length.")
-        self._ensure_rows(B * N)
+        pm = self._packed(self._device)
+        self._ensure_rows(B * N, pm)
         x = embedding.detach().to(torch.float32).contiguous()
         z = torch.empty(B, N, D, device=embedding.device, dtype=torch.float32)
-        pm = self._packed(self._device)
         self._state.buffer_len = self.buffer_len
         _lib.check(lib.artab_decode_embedded(pm.ref, C.byref(self._state), _lib.ptr(x), N, commit, _lib.ptr(z),
                                              _lib.stream_ptr()))
@@ -363,7 +382,8 @@ class ARTabPFNPredictor:
             expo = torch.empty(Nt, B, K, device=device, dtype=torch.float32)     # owned by the main stream
             normal = torch.empty(Nt, B, device=device, dtype=torch.float32)
             fresh = main.record_event()      # whatever used this memory before has finished by here
-        self.prefill_context(x_context, y_context)
+        pm = self._packed(self._device)
+        self._prefill(x_context, y_context, pm)
         if variates is None:
             side.wait_event(fresh)
             drawn = {}
@@ -388,7 +408,6 @@ class ARTabPFNPredictor:
         samples = torch.empty(B, Nt, device=device, dtype=torch.float32)
         logdens = torch.empty(B, Nt, device=device, dtype=torch.float32)
         comp = torch.empty(B, Nt, device=device, dtype=torch.int32)
-        pm = self._packed(device)
         st = self._state
         stream = _lib.stream_ptr()
 
@@ -442,12 +461,12 @@ class ARTabPFNPredictor:
         else:
             # the reference reserves Nc + 2*Nt; only the Nt buffer rows are ever cached
             self.init_kv_cache(B, Nc + Nt, device, dtype)
-        self.prefill_context(x_context, y_context)
-        self._ensure_rows(2 * B * Nt)
+        pm = self._packed(self._device)
+        self._prefill(x_context, y_context, pm)
+        self._ensure_rows(2 * B * Nt, pm)
         xt = self._dev32(x_target, device)
         yt = self._dev32(y_target, device).reshape(B, Nt)
         out = torch.empty(B, Nt, device=device, dtype=torch.float32)
-        pm = self._packed(device)
         _lib.check(lib.artab_teacher_forcing(pm.ref, C.byref(self._state), _lib.ptr(xt), _lib.ptr(yt), F, Nt,
                                              _lib.ptr(out), _lib.stream_ptr()))
         self.buffer_len = int(self._state.buffer_len)
@@ -477,14 +496,14 @@ class ARTabPFNPredictor:
             self.init_kv_cache(B, Nb, device, dtype)
         else:
             self.init_kv_cache(B, Nc + Nb, device, dtype)
-        self.prefill_context(x_context, y_context)
-        self._ensure_rows(B * (Nb + Nt))
+        pm = self._packed(self._device)
+        self._prefill(x_context, y_context, pm)
+        self._ensure_rows(B * (Nb + Nt), pm)
         f32 = lambda t, *shape: self._dev32(t, device).reshape(*shape)
         xb, yb = f32(x_buffer, B, Nb, F), f32(y_buffer, B, Nb)
         xt, yt = f32(x_target, B, Nt, F), f32(y_target, B, Nt)
         vis = torch.tensor([int(v) for v in visible], dtype=torch.int32, device=device)
         out = torch.empty(B, Nt, device=device, dtype=torch.float32)
-        pm = self._packed(device)
         _lib.check(lib.artab_forward_masked(pm.ref, C.byref(self._state), _lib.ptr(xb), _lib.ptr(yb), _lib.ptr(xt),
                                             _lib.ptr(yt), F, Nb, Nt, _lib.ptr(vis), _lib.ptr(out),
                                             _lib.stream_ptr()))

@@ -54,3 +54,22 @@ def test_bf16_joint_density_at_row_edges(case):
     ld = pred.last_logdens.clone()
     gap = (pred.evaluate_joint_density(*(t.cuda() for t in args[:3]), ys) - ld).abs()
     assert bool(torch.isfinite(ys).all()) and float(gap.median()) <= 2e-3
+
+
+@pytest.mark.parametrize("precision", ["fp32", "bf16"])
+def test_layouts_in_turn_on_one_predictor(precision):
+    """Context lengths with and without padding of the key axis, in turn on one predictor whose buffers are reused:
+    the same bits as a predictor of its own gives."""
+    import ar_tabpfn
+    torch.manual_seed(3)
+    m = ar_tabpfn.ARTabPFN(d_model=64, n_heads=2, n_layers=2, d_ff=128, num_features=4).eval().cuda()
+    make = lambda: ar_tabpfn.ARTabPFNPredictor.from_trained_model(m, backend="flex_attention", precision=precision)
+    kept, other = make(), make()
+    for Nc, B, Nt in ((50, 3, 6), (43, 3, 6), (43, 3, 6), (50, 3, 6), (50, 2, 9), (48, 3, 6)):
+        g = torch.Generator(device="cuda").manual_seed(Nc + B)
+        x, y = torch.randn(B, Nc + Nt, 4, generator=g, device="cuda"), torch.randn(B, Nc + Nt, generator=g, device="cuda")
+        args = (x[:, :Nc], y[:, :Nc], x[:, Nc:], y[:, Nc:])
+        got = kept.evaluate_joint_density(*args)
+        assert m.backbone.layers[1].k_ctx_cache.shape[2] == Nc
+        other.evaluate_joint_density(*args)   # takes the modules' cache views for itself
+        assert torch.equal(got, make().evaluate_joint_density(*args))
