@@ -47,10 +47,10 @@ import synthetic as syn  # noqa: E402
 
 CFG = dict(syn.MODEL_6L, num_features=syn.CONFIG3["num_features"])
 NC, NT, STREAMS, SEED = syn.CONFIG3["n_ctx"], syn.CONFIG3["n_targets"], syn.CONFIG3["streams"], syn.CONFIG3["seed"]
-# DRAM bytes (read + write) of one 1024-row decode-step launch of the tensor-core dense chain: a constant
+# DRAM bytes (read + write) of one 1024-row decode-step launch of the bf16 dense chain (dense_mma_kernel): a constant
 # taken from one ncu capture of that kernel (dram__bytes_read.sum + dram__bytes_write.sum), not measured
 # in this run; the weight tiles dominate it
-DENSE_TC_DRAM_BYTES_PER_LAUNCH = 3.68e6
+DENSE_DRAM_BYTES_PER_LAUNCH = 5.07e6
 CPU_SAMPLE = dict(streams=128, targets=16)  # bounded CPU sample of the same workload
 WORKLOAD_CONFIG = {"workload": "config3: 6L d192 h6 ff768, ctx 1024x20, 128 targets, 512 streams/GPU, "
                                "shared context KV, prefill included in every step",
@@ -424,14 +424,14 @@ def main():
             peak = peaks.get("bf16_tflops_sustained", 1400.0)
             ach = flops / (shares[dom]["ms"] * 1e-3) / 1e12
             tc = args.precision == "bf16"
-            roof = {"kernel": "dense_tc_kernel" if tc else "dense_chain_kernel", "bound": "tensor",
+            roof = {"kernel": "dense_mma_kernel" if tc else "dense_fma_kernel", "bound": "tensor",
                     "achieved": ach, "peak": peak, "unit": "TFLOP/s", "frac": ach / peak,
-                    "traffic": DENSE_TC_DRAM_BYTES_PER_LAUNCH if tc else None,
+                    "traffic": DENSE_DRAM_BYTES_PER_LAUNCH if tc else None,
                     "traffic_source": "constant: DRAM bytes of one 1024-row decode launch in an ncu capture, "
                                       "not measured in this run" if tc else None,
                     "peak_source": "measured" if peaks else "fallback",
-                    "note": ("tcgen05 chain, 8 row tiles of 128 rows per decode launch: bound by the latency of the "
-                             "dependent GEMM / LayerNorm chain of a row tile, not by the tensor pipe"
+                    "note": ("32 clusters of four CTAs over 32 rows per decode launch: bound by the latency of the "
+                             "dependent product / LayerNorm / exchange phases, not by the tensor pipe"
                              if tc else "fp32 FMA kernel measured against the bf16 tensor peak")}
         elif dom == "context_attention":
             q_rows = STREAMS * (1 + 2 * (NT - 1)) + NC
