@@ -16,11 +16,13 @@ CASES = [
     (64, 1, 1, 64, 5, 3, 64, 5, True),          # one head: no cluster to form, the launch-per-layer path
     (128, 4, 2, 256, 5, 130, 40, 4, True),      # four streams per cluster, the last cluster not full
     (128, 2, 1, 256, 3, 9, 70, 5, False),       # head size 64, own contexts
-    (128, 8, 1, 512, 5, 200, 30, 3, True),      # eight CTAs, many streams: the widest variant
+    (128, 8, 1, 512, 5, 200, 30, 3, True),      # eight CTAs, more streams than one wave: the launch-per-layer path
     (192, 6, 1, 768, 5, 20, 65, 4, False),      # own contexts, head size 32
     (192, 12, 1, 192, 5, 3, 20, 3, True),       # two heads of 16 per CTA
     (64, 4, 1, 128, 5, 6, 50, 140, True),       # private keys beyond one round of the four parts
-    (64, 4, 1, 128, 5, 420, 20, 3, False),      # more streams than one wave of clusters holds
+    (128, 8, 1, 512, 5, 100, 30, 3, True),      # eight CTAs, the widest variant within one wave
+    (64, 4, 1, 128, 8, 250, 20, 3, False),      # the widest variant, a context per stream, clusters not full
+    (64, 4, 1, 128, 5, 420, 20, 3, False),      # the same with a context per stream
 ]
 
 
