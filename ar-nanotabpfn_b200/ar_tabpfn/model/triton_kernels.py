@@ -274,20 +274,52 @@ def pytorch_context_attention(q: Tensor, k_ctx: Tensor, v_ctx: Tensor,
     return triton_context_attention(q, k_ctx, v_ctx, scale=scale)
 
 
+def _hybrid_grouped(q: Tensor, k_ctx: Tensor, v_ctx: Tensor, k_buf: Tensor, v_buf: Tensor,
+                    buf_mask: Optional[Tensor]) -> Tensor:
+    """``hybrid_attention`` for a context per stream ([B,H,Nc,Dh]) and for a V that broadcasts to the shape of K:
+    packed K / V, per-group contraction.  Shapes that do not fit raise while packing or in the library's checks."""
+    B, H, Lq, Dh = q.shape
+    Nb = k_buf.shape[2]
+    lib = _lib.lib()
+    lens = _stream_lengths(buf_mask, B, H, Lq, Nb, q.device) if buf_mask is not None else None
+    k, v, Nc, Ncp = pack_context(k_ctx.to(q.dtype), v_ctx.to(q.dtype))
+    kv = _pack_buffer(k_buf.to(q.dtype), v_buf.to(q.dtype))
+
+    def context(qr, n):
+        splits = lib.artab_plan_splits(_lib.dtype_code(q.dtype), B * n, n, 1, H, Nc)
+        o, l = _context_partials(qr, k, v, Nc, Ncp, n if k.shape[0] > 1 else B * n, splits)
+        return o, l, splits
+
+    if buf_mask is not None and lens is None:
+        return _buffer_merge_masked(q, kv, buf_mask, context, want_lse=False)[0].to(q.dtype)
+    return _buffer_merge(q, kv, lens, context, want_lse=False)[0].to(q.dtype)
+
+
 def hybrid_attention(q: Tensor, k_ctx: Tensor, v_ctx: Tensor, k_buf: Tensor, v_buf: Tensor,
                      buf_mask: Optional[Tensor] = None, use_triton: bool = True) -> Tensor:
     """Shared-context attention + private-buffer attention merged by log-sum-exp.  Every query
     sees every buffer key of its stream, or with ``buf_mask`` (any boolean tensor broadcastable to
-    [B,H,Lq,Nb]) what the mask lets it see.  Returns [B,H,Lq,Dh]."""
+    [B,H,Lq,Nb]) what the mask lets it see.  The context may also be [1,H,Nc,Dh], or [B,H,Nc,Dh] for
+    one per stream.  Returns [B,H,Lq,Dh]."""
     B, H, Lq, Dh = q.shape
     Nb = k_buf.shape[2]
     if Nb == 0:
         return triton_context_attention(q, k_ctx, v_ctx)[0]
+    if any(t.device != q.device for t in (k_ctx, v_ctx, k_buf, v_buf)):
+        raise ValueError("hybrid_attention: all tensors must live on the device of q")
+    # The kernels see addresses and the sizes of q and K: every extent is checked here.
+    if tuple(k_buf.shape) != (B, H, Nb, Dh):
+        raise ValueError(f"hybrid_attention: k_buf {tuple(k_buf.shape)} does not fit q {tuple(q.shape)}")
+    if k_ctx.dim() not in (3, 4) or k_ctx.shape[-3] != H or k_ctx.shape[-1] != Dh:
+        raise ValueError(f"hybrid_attention: k_ctx {tuple(k_ctx.shape)} does not fit q {tuple(q.shape)}")
+    if k_ctx.dim() == 4 and k_ctx.shape[0] == 1 and v_ctx.shape == k_ctx.shape:
+        k_ctx, v_ctx = k_ctx[0], v_ctx[0]
+    if k_ctx.dim() == 4 or v_ctx.shape != k_ctx.shape or v_buf.shape != k_buf.shape:
+        return _hybrid_grouped(q, k_ctx, v_ctx, k_buf, v_buf, buf_mask)
     lib = _lib.lib()
     code = _lib.dtype_code(q.dtype)
     # token-major queries: with one query per stream that is the tensor itself
-    qr = _plain(q, q.dtype) if Lq == 1 else _rows(q)
-    kc, vc, kb, vb = (_plain(t, q.dtype) for t in (k_ctx, v_ctx, k_buf, v_buf))
+    qr, kc, vc, kb, vb = (_plain(t, q.dtype) for t in (q if Lq == 1 else _rows(q), k_ctx, v_ctx, k_buf, v_buf))
     strides = None
     if buf_mask is not None:
         if buf_mask.device != q.device or buf_mask.dtype != torch.bool:

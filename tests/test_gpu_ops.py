@@ -368,3 +368,27 @@ def test_hybrid_attention_masks_and_tile_edges(shape, dtype):
         # averaged over the keys); fp32: sums over up to 2088 keys
         rel = float((got.float() - want).norm() / want.norm())
         assert rel <= (2 ** -8 if dtype == torch.bfloat16 else 1e-5), rel
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("mask", [None, "prefix", "any"])
+def test_hybrid_attention_with_a_context_per_stream(tk, mask, dtype):
+    """[B,H,Nc,Dh] contexts, one per stream, and the [1,H,Nc,Dh] form of a shared one; [1,Nc,Dh] V for all heads."""
+    B, H, Lq, Nc, Nb, Dh = 5, 3, 2, 37, 21, 32
+    g = torch.Generator(device="cuda").manual_seed(11)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).to(dtype)
+    q, kc, vc, kb, vb = r(B, H, Lq, Dh), r(B, H, Nc, Dh), r(B, H, Nc, Dh), r(B, H, Nb, Dh), r(B, H, Nb, Dh)
+    m = None
+    if mask == "prefix":
+        m = (torch.arange(Nb, device="cuda")[None] < torch.tensor([0, 1, 7, 20, 21], device="cuda")[:, None]).view(B, 1, 1, Nb)
+    elif mask == "any":
+        m = torch.rand(B, H, Lq, Nb, device="cuda", generator=g) < 0.4
+    full = torch.ones(B, H, Lq, Nc + Nb, dtype=torch.bool, device="cuda")
+    if m is not None:
+        full[..., Nc:] = m
+    tol = 1e-5 if dtype == torch.float32 else 1e-2
+    for k, v in ((kc, vc), (kc[:1], vc[:1]), (kc[0], vc[0, :1])):
+        got = tk.hybrid_attention(q, k, v, kb, vb, buf_mask=m).float()
+        wide = lambda t: t.expand(B, H, Nc, Dh)
+        want, _ = ref_attention(q, torch.cat([wide(k), kb], 2), torch.cat([wide(v), vb], 2), full)
+        assert float((got - want).abs().max() / want.abs().max()) <= tol
