@@ -19,6 +19,7 @@ from .. import _lib
 
 
 last_status = None
+_Strides = C.c_int64 * 4
 
 
 def triton_available() -> bool:
@@ -30,23 +31,10 @@ def triton_available() -> bool:
         return False
 
 
-_STATUS = {}
-
-
-def _status_word(device) -> Tensor:
-    """The device's status word of the calls that do not allocate one each time: zero until a bounded
-    device-side wait gives up (that call's result is NaN); also kept in ``last_status``."""
-    global last_status
-    t = _STATUS.get(device)
-    if t is None:
-        t = _STATUS[device] = torch.zeros(1, device=device, dtype=torch.int32)
-    last_status = t
-    return t
-
-
 def _plain(t: Tensor, dtype) -> Tensor:
     """``t`` as a contiguous, 16-byte aligned tensor of ``dtype``: itself when it already is one."""
-    t = t.to(dtype).contiguous()
+    if t.dtype is not dtype or not t.is_contiguous():
+        t = t.to(dtype).contiguous()
     return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
@@ -305,16 +293,19 @@ def hybrid_attention(q: Tensor, k_ctx: Tensor, v_ctx: Tensor, k_buf: Tensor, v_b
     Nb = k_buf.shape[2]
     if Nb == 0:
         return triton_context_attention(q, k_ctx, v_ctx)[0]
-    if any(t.device != q.device for t in (k_ctx, v_ctx, k_buf, v_buf)):
-        raise ValueError("hybrid_attention: all tensors must live on the device of q")
     # The kernels see addresses and the sizes of q and K: every extent is checked here.
-    if tuple(k_buf.shape) != (B, H, Nb, Dh):
+    dev = q.get_device()
+    if not k_ctx.get_device() == v_ctx.get_device() == k_buf.get_device() == v_buf.get_device() == dev:
+        raise ValueError("hybrid_attention: all tensors must live on the device of q")
+    if k_buf.shape != (B, H, Nb, Dh):
         raise ValueError(f"hybrid_attention: k_buf {tuple(k_buf.shape)} does not fit q {tuple(q.shape)}")
-    if k_ctx.dim() not in (3, 4) or k_ctx.shape[-3] != H or k_ctx.shape[-1] != Dh:
-        raise ValueError(f"hybrid_attention: k_ctx {tuple(k_ctx.shape)} does not fit q {tuple(q.shape)}")
-    if k_ctx.dim() == 4 and k_ctx.shape[0] == 1 and v_ctx.shape == k_ctx.shape:
-        k_ctx, v_ctx = k_ctx[0], v_ctx[0]
-    if k_ctx.dim() == 4 or v_ctx.shape != k_ctx.shape or v_buf.shape != k_buf.shape:
+    Nc = k_ctx.shape[-2]
+    if k_ctx.shape != (H, Nc, Dh):
+        if k_ctx.dim() != 4 or k_ctx.shape[1:] != (H, Nc, Dh):
+            raise ValueError(f"hybrid_attention: k_ctx {tuple(k_ctx.shape)} does not fit q {tuple(q.shape)}")
+        if k_ctx.shape[0] == 1 and v_ctx.shape == k_ctx.shape:
+            k_ctx, v_ctx = k_ctx[0], v_ctx[0]
+    if v_ctx.shape != (H, Nc, Dh) or k_ctx.dim() == 4 or v_buf.shape != k_buf.shape:
         return _hybrid_grouped(q, k_ctx, v_ctx, k_buf, v_buf, buf_mask)
     lib = _lib.lib()
     code = _lib.dtype_code(q.dtype)
@@ -322,18 +313,19 @@ def hybrid_attention(q: Tensor, k_ctx: Tensor, v_ctx: Tensor, k_buf: Tensor, v_b
     qr, kc, vc, kb, vb = (_plain(t, q.dtype) for t in (q if Lq == 1 else _rows(q), k_ctx, v_ctx, k_buf, v_buf))
     strides = None
     if buf_mask is not None:
-        if buf_mask.device != q.device or buf_mask.dtype != torch.bool:
+        if buf_mask.get_device() != dev or buf_mask.dtype is not torch.bool:
             buf_mask = buf_mask.to(device=q.device, dtype=torch.bool)
         buf_mask = buf_mask.expand(B, H, Lq, Nb)
-        strides = (C.c_int64 * 4)(*buf_mask.stride())
-    Nc = kc.shape[1]
-    need = int(lib.artab_hybrid_workspace(code, B, H, Lq, Dh, Nc))
-    ws = torch.empty(need, dtype=torch.uint8, device=q.device)
-    out = torch.empty(B, H, Lq, Dh, dtype=q.dtype, device=q.device)
+        strides = _Strides(*buf_mask.stride())
+    need = lib.artab_hybrid_workspace(code, B, H, Lq, Dh, Nc)
+    device = q.device
+    ws = torch.empty(need, dtype=torch.uint8, device=device)
+    out = torch.empty((B, H, Lq, Dh), dtype=q.dtype, device=device)
+    global last_status
+    last_status = status = torch.empty(1, dtype=torch.int32, device=device)  # written by this call
     _lib.check(lib.artab_hybrid_attention(
         code, qr.data_ptr(), kc.data_ptr(), vc.data_ptr(), kb.data_ptr(), vb.data_ptr(), _lib.ptr(buf_mask), strides,
-        B, H, Lq, Dh, Nc, Nb, out.data_ptr(), ws.data_ptr(), need, _status_word(q.device).data_ptr(),
-        _lib.stream_ptr()))
+        B, H, Lq, Dh, Nc, Nb, out.data_ptr(), ws.data_ptr(), need, status.data_ptr(), _lib.stream_ptr()))
     return out
 
 

@@ -896,7 +896,8 @@ static int hybrid_splits(int dtype, int rows, int n_heads, int head_dim, int n_c
 }
 int64_t artab_hybrid_workspace(int dtype, int n_streams, int n_heads, int n_q, int head_dim, int n_ctx) {
   const int rows = n_streams * n_q;
-  return (int64_t)hybrid_splits(dtype, rows, n_heads, head_dim, n_ctx) * rows * n_heads * (head_dim + 1) * 4;
+  const int splits = hybrid_splits(dtype, rows, n_heads, head_dim, n_ctx);
+  return 4 * ((int64_t)splits * rows * n_heads * (head_dim + 1) + ctx_attn_tc_ctas(rows, n_heads, splits));
 }
 
 int artab_hybrid_attention(int dtype, const void* q, const void* k_ctx, const void* v_ctx, const void* k_buf,
@@ -933,11 +934,13 @@ int artab_hybrid_attention(int dtype, const void* q, const void* k_ctx, const vo
   c.scale = 1.0f / sqrtf((float)head_dim);
   c.out = (float*)workspace;
   c.lse = c.out + (size_t)c.n_splits * rows * n_heads * head_dim;
-  c.status = status;
+  // a status per CTA: there is no word to clear, and nothing of an earlier or concurrent call is read
+  const bool tc = use_tc(dtype, head_dim);
+  c.cta_status = tc ? (int32_t*)(c.lse + (size_t)c.n_splits * rows * n_heads) : nullptr;
   int rc;
   {
     PlainLaunchScope plain;  // the caller's earlier launches are unknown: see common.cuh
-    rc = use_tc(dtype, head_dim) ? launch_ctx_attn_tc(c, s) : launch_ctx_attn_simt(c, s);
+    rc = tc ? launch_ctx_attn_tc(c, s) : launch_ctx_attn_simt(c, s);
   }
   if (rc) return rc;
   // The merge may start beside the contraction: what it reads before its wait (queries, private K / V, mask)
@@ -967,7 +970,9 @@ int artab_hybrid_attention(int dtype, const void* q, const void* k_ctx, const vo
   b.n_splits = c.n_splits;
   b.rows = rows;
   b.scale = c.scale;
-  b.poison_if = status;
+  b.cta_status = c.cta_status;
+  b.n_cta_status = tc ? ctx_attn_tc_ctas(rows, n_heads, c.n_splits) : 0;
+  b.op_status = status;
   return launch_hybrid_merge(b, s);
 }
 

@@ -16,6 +16,9 @@ struct CtxAttnArgs {
   int out_lane_major; // n_splits == 1 only: write the [rows][H*Dh] result in the lane-major layout
   float* lse;         // [splits][rows][H]
   int32_t* status;    // device status word (bounded waits), may be null for SIMT
+  // Optional, tensor-core kernel: every CTA stores 0, or 1 when one of its waits gave up (its rows then have an LSE of
+  // +inf, which makes their merged result NaN).  ctx_attn_tc_ctas words that need no clearing beforehand.
+  int32_t* cta_status;
   int kv_stable;      // k_ctx / v_ctx were not written by the kernel launched just before this one
 };
 
@@ -36,6 +39,9 @@ struct BufMergeArgs {
   int op_q;
   long ms_b, ms_h, ms_q, ms_k;
   void* op_out;
+  const int32_t* cta_status;  // CtxAttnArgs::cta_status of the contraction, n_cta_status words
+  int n_cta_status;
+  int32_t* op_status;         // optional: 0, or 1 when a wait of the contraction gave up
   const int32_t* lens;     // mode 0: [B] visible buffer rows of each stream, clamped to len0 (null: len0 for all)
   float* lse_out;          // optional [rows][H]: natural-log LSE of the merged attention (-inf: nothing visible)
   long n_items;
@@ -55,6 +61,7 @@ int launch_ctx_attn_simt(const CtxAttnArgs& a, cudaStream_t s);  // fp32 FMA, he
 int ctx_attn_fma_rows(int rows_in_group);                        // query rows of one of its CTAs
 int launch_ctx_attn_tc(const CtxAttnArgs& a, cudaStream_t s);  // tcgen05, bf16, head_dim 32
 bool ctx_attn_tc_supported(int dtype, int head_dim);
+int ctx_attn_tc_ctas(int rows, int n_heads, int n_splits);        // CTAs of a launch on one shared context
 int launch_buf_merge(const BufMergeArgs& a, cudaStream_t s);      // picks the MMA kernel when it applies
 int launch_buf_merge_mma(const BufMergeArgs& a, cudaStream_t s);  // mma.sync, bf16, head_dim 32
 bool buf_mma_supported(int dtype, int head_dim);

@@ -201,6 +201,15 @@ __global__ void __launch_bounds__(128, 6) buf_merge_kernel(const BufMergeArgs a)
   // The buffer pass above read only what kernels older than the preceding one wrote (q and the
   // buffer rows); the context partials come from the preceding kernel.
   dep_wait();
+  if constexpr (OP) {   // one warp gathers what the CTAs of the contraction report: no word has to be cleared
+    if (item == 0 && a.op_status) {
+      int bad = 0;
+#pragma unroll 8
+      for (int i = lane; i < a.n_cta_status; i += 32) bad |= __ldcg(a.cta_status + i);
+      bad = __any_sync(0xffffffffu, bad != 0);
+      if (lane == 0) *a.op_status = bad;
+    }
+  }
 
   // log-sum-exp merge with the context partials, all in registers
 #pragma unroll

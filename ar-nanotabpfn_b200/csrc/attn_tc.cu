@@ -228,6 +228,7 @@ struct TcParams {
   float* out;
   float* lse;
   int32_t* status;
+  int32_t* cta_status;
   long long wait_cycles;  // limit of every mbarrier wait, in SM clock cycles
   int drop_score_commits; // diagnostics only: the MMA thread never signals "scores ready", so the waits run out
 };
@@ -444,6 +445,7 @@ ctx_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       for (int i = 0; i < DH / 4; ++i) o[i] = make_float4(0.f, 0.f, 0.f, 0.f);
       p.lse[out_row] = -INFINITY;
     }
+    if (threadIdx.x == 0 && p.cta_status) p.cta_status[(blockIdx.z * gridDim.y + h) * gridDim.x + blockIdx.x] = 0;
     return;
   }
 
@@ -670,6 +672,10 @@ ctx_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
   }
   if (threadIdx.x == 0 && sm->ctl.abort_flag && p.status) atomicExch(p.status, 1);
+  if (p.cta_status) {
+    if (threadIdx.x == 0) p.cta_status[(blockIdx.z * gridDim.y + h) * gridDim.x + blockIdx.x] = sm->ctl.abort_flag ? 1 : 0;
+    if (sm->ctl.abort_flag && row_valid) p.lse[out_row] = INFINITY;
+  }
   if (threadIdx.x == 0) ARTAB_STAMP(2, 2);
 }
 
@@ -742,6 +748,8 @@ int make_map_2d(CUtensorMap* tm, const void* base, uint64_t inner, uint64_t oute
 
 bool ctx_attn_tc_supported(int dtype, int head_dim) { return dtype == ARTAB_BF16 && head_dim == DH; }
 
+int ctx_attn_tc_ctas(int rows, int n_heads, int n_splits) { return (rows + BM - 1) / BM * n_heads * n_splits; }
+
 int launch_ctx_attn_tc(const CtxAttnArgs& a, cudaStream_t s) {
   if (a.rows <= 0) return ARTAB_OK;
   ARTAB_REQUIRE(a.dtype == ARTAB_BF16 && a.head_dim == DH && (a.v_transposed || a.n_groups == 1), ARTAB_EINVAL,
@@ -791,6 +799,7 @@ int launch_ctx_attn_tc(const CtxAttnArgs& a, cudaStream_t s) {
   p.out = a.out;
   p.lse = a.lse;
   p.status = a.status;
+  p.cta_status = a.cta_status;
   p.wait_cycles = debug_wait_cycles() > 0 ? debug_wait_cycles() : kWaitCycles;
   p.drop_score_commits = debug_drop_score_commits();
   const int rows_in_group = a.n_groups == 1 ? a.rows : a.rows_per_group;

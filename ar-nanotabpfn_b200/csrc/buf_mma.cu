@@ -232,6 +232,15 @@ __global__ void __launch_bounds__(WPB * 32, 6) buf_mma_kernel(const BufMergeArgs
   if (threadIdx.x == 0) ARTAB_STAMP(3, 3);
   dep_wait();
   if (threadIdx.x == 0) ARTAB_STAMP(3, 1);
+  if constexpr (OP) {   // one warp gathers what the CTAs of the contraction report: no word has to be cleared
+    if (item == 0 && a.op_status) {
+      int bad = 0;
+#pragma unroll 8
+      for (int i = lane; i < a.n_cta_status; i += 32) bad |= __ldcg(a.cta_status + i);
+      bad = __any_sync(0xffffffffu, bad != 0);
+      if (lane == 0) *a.op_status = bad;
+    }
+  }
 
   if (g >= 2 || rows2[g & 1] < 0) return;
   const long r = rows2[g];

@@ -341,7 +341,8 @@ ARTAB_API int artab_buffer_attention_merge_ragged(int dtype, const void* q, cons
  *   q [B*Lq][H][Dh] (token-major; the reference's [B,H,1,Dh] as it is when Lq = 1); k_ctx / v_ctx [H][Nc][Dh];
  *   k_buf / v_buf [B][H][Nb][Dh]; mask: one byte per key, non-zero = visible, element (b, h, l, key) at
  *   mask + sum of index * mask_strides[i] (HOST array of four, 0 broadcasts), or NULL: every key visible;
- *   out [B][H][Lq][Dh] of the input type; workspace of artab_hybrid_workspace bytes.
+ *   out [B][H][Lq][Dh] of the input type; workspace of artab_hybrid_workspace bytes;
+ *   status: written by this call (or NULL): 0, or 1 when a bounded wait gave up, upon which the rows of out it concerns are NaN.
  * Replaces hybrid_attention (ar_tabpfn/model/triton_kernels.py:662-708). */
 ARTAB_API int64_t artab_hybrid_workspace(int dtype, int n_streams, int n_heads, int n_q, int head_dim, int n_ctx);
 ARTAB_API int artab_hybrid_attention(int dtype, const void* q, const void* k_ctx, const void* v_ctx, const void* k_buf,

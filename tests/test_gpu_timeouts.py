@@ -86,6 +86,35 @@ def test_noalloc_entry_reports_a_timed_out_wait_as_nan():
     assert torch.equal(out, good)
 
 
+def test_hybrid_attention_timed_out_call_is_nan_and_the_next_one_is_not():
+    from ar_tabpfn import _lib
+    from ar_tabpfn.model import triton_kernels as tk
+    lib = _lib.lib()
+    g = torch.Generator(device="cuda").manual_seed(3)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    args = r(70, 2, 1, 32), r(2, 300, 32), r(2, 300, 32), r(70, 2, 9, 32), r(70, 2, 9, 32)
+    good = tk.hybrid_attention(*args)
+    assert int(tk.last_status.item()) == 0
+    try:
+        _lib.check(lib.artab_debug_set(_lib.DEBUG_WAIT_CYCLES, 200_000))
+        _lib.check(lib.artab_debug_set(_lib.DEBUG_DROP_SCORE_COMMITS, 1))
+        bad = tk.hybrid_attention(*args)
+        torch.cuda.synchronize()
+    finally:
+        lib.artab_debug_set(_lib.DEBUG_DROP_SCORE_COMMITS, 0)
+        lib.artab_debug_set(_lib.DEBUG_WAIT_CYCLES, 0)
+    word = tk.last_status
+    assert int(word.item()) != 0 and bool(torch.isnan(bad).all())
+    assert torch.equal(tk.hybrid_attention(*args), good)      # every call has a word of its own ...
+    assert int(tk.last_status.item()) == 0 and int(word.item()) != 0
+    # ... written by the call itself, whatever its memory held before
+    q, k, v, kb, vb = args
+    out, ws = torch.empty_like(q), torch.empty(1 << 20, dtype=torch.uint8, device="cuda")
+    _lib.check(lib.artab_hybrid_attention(_lib.BF16, *(_lib.ptr(t) for t in args), None, None, 70, 2, 1, 32, 300, 9,
+                                          _lib.ptr(out), _lib.ptr(ws), ws.numel(), _lib.ptr(word), _lib.stream_ptr()))
+    assert torch.equal(out, good) and int(word.item()) == 0
+
+
 def test_predictor_raises_after_a_timed_out_call():
     from ar_tabpfn import _lib
     from ar_tabpfn.model import ARTabPFNPredictor
