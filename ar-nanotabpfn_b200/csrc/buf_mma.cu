@@ -2,7 +2,8 @@
 //
 // Same job and the same one-warp-per-(stream, head[, item]) mapping as buf_merge_kernel, but the two
 // queries of an item are rows 0 and 1 of an m16n8k16 A fragment, so a block of 16 keys costs
-// 4 (Q.K^T) + 8 (P.V with P split into bf16 hi + lo, which keeps P at fp32 accuracy) MMAs and a
+// 4 (Q.K^T) + 8 (P.V with P split into bf16 hi + lo, 16 bits, or in the operator form into three parts,
+// 24 bits: its masked calls once ran in fp32 FMA) MMAs and a
 // two-value softmax per lane instead of ~140 scalar instructions.  A key's K row and V row are
 // adjacent in memory, so a block of 16 keys is one contiguous 2 KB span: it goes through a 4-slot
 // shared-memory ring filled with 16-byte cp.async copies and is read with ldmatrix (K^T fragments)
@@ -23,12 +24,13 @@ constexpr int WPB = 4;     // warps per CTA
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
-  // rows 8-15 of A (fragment registers a1, a3) are always zero here: only two query rows exist
+// a1, a3: rows 8-15 of A, zero unless given: only two query rows exist
+__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1, uint32_t a1 = 0u,
+                                         uint32_t a3 = 0u) {
   asm volatile(
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a0), "r"(0u), "r"(a2), "r"(0u), "r"(b0), "r"(b1));
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t saddr, uint32_t (&r)[4]) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -152,7 +154,7 @@ __global__ void __launch_bounds__(WPB * 32, 6) buf_mma_kernel(const BufMergeArgs
   };
 
   float m = -INFINITY, l = 0.f;
-  float o[4][4];  // [8-dim tile][c0..c3]: c0, c1 = row g, dims tile*8 + t4*2 + {0,1}; c2, c3 stay zero
+  float o[4][4];  // [8-dim tile][c0..c3]: c0, c1 = row g, dims tile*8 + t4*2 + {0,1}; c2, c3: OP the middle part of P, else zero
 #pragma unroll
   for (int j = 0; j < 4; ++j)
 #pragma unroll
@@ -206,21 +208,36 @@ __global__ void __launch_bounds__(WPB * 32, 6) buf_mma_kernel(const BufMergeArgs
     for (int j = 0; j < 4; ++j) {
       o[j][0] *= alpha;
       o[j][1] *= alpha;
+      if constexpr (OP) {
+        o[j][2] *= alpha;
+        o[j][3] *= alpha;
+      }
     }
     // P as the A operand of P.V (k = 16 keys): a0 = keys t4*2+{0,1}, a2 = the same + 8; hi + lo parts
     const uint32_t ph0 = pack_bf16(p[0], p[1]), ph1 = pack_bf16(p[2], p[3]);
-    const uint32_t pl0 = pack_bf16(p[0] - __uint_as_float(ph0 << 16), p[1] - __uint_as_float(ph0 & 0xffff0000u));
-    const uint32_t pl1 = pack_bf16(p[2] - __uint_as_float(ph1 << 16), p[3] - __uint_as_float(ph1 & 0xffff0000u));
+    const float r0 = p[0] - __uint_as_float(ph0 << 16), r1 = p[1] - __uint_as_float(ph0 & 0xffff0000u);
+    const float r2 = p[2] - __uint_as_float(ph1 << 16), r3 = p[3] - __uint_as_float(ph1 & 0xffff0000u);
+    const uint32_t pl0 = pack_bf16(r0, r1), pl1 = pack_bf16(r2, r3);
+    [[maybe_unused]] const uint32_t pt0 = pack_bf16(r0 - __uint_as_float(pl0 << 16), r1 - __uint_as_float(pl0 & 0xffff0000u));
+    [[maybe_unused]] const uint32_t pt1 = pack_bf16(r2 - __uint_as_float(pl1 << 16), r3 - __uint_as_float(pl1 & 0xffff0000u));
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
       // V fragments (ldmatrix.trans of [8 keys][8 dims] blocks of the V half of the staged rows):
       // (dim tile 2c, keys 0-7), (2c, keys 8-15), (2c+1, keys 0-7), (2c+1, keys 8-15)
       uint32_t vb[4];
       ldmatrix_x4_trans(slot + (uint32_t)(((mi & 1) * 8 + r8) * PITCH + 64 + (2 * c + (mi >> 1)) * 16), vb);
-      mma_bf16(o[2 * c], ph0, ph1, vb[0], vb[1]);
-      mma_bf16(o[2 * c], pl0, pl1, vb[0], vb[1]);
-      mma_bf16(o[2 * c + 1], ph0, ph1, vb[2], vb[3]);
-      mma_bf16(o[2 * c + 1], pl0, pl1, vb[2], vb[3]);
+      if constexpr (OP) {
+        // P as three parts, which is all of its 24 bits, in as many MMAs: the empty rows 8-15 take the second part
+        mma_bf16(o[2 * c], ph0, ph1, vb[0], vb[1], pl0, pl1);
+        mma_bf16(o[2 * c], pt0, pt1, vb[0], vb[1]);
+        mma_bf16(o[2 * c + 1], ph0, ph1, vb[2], vb[3], pl0, pl1);
+        mma_bf16(o[2 * c + 1], pt0, pt1, vb[2], vb[3]);
+      } else {
+        mma_bf16(o[2 * c], ph0, ph1, vb[0], vb[1]);
+        mma_bf16(o[2 * c], pl0, pl1, vb[0], vb[1]);
+        mma_bf16(o[2 * c + 1], ph0, ph1, vb[2], vb[3]);
+        mma_bf16(o[2 * c + 1], pl0, pl1, vb[2], vb[3]);
+      }
     }
   }
   cp_async_wait<0>();
@@ -253,8 +270,8 @@ __global__ void __launch_bounds__(WPB * 32, 6) buf_mma_kernel(const BufMergeArgs
     const float inv = l > 0.f ? 1.0f / l : 0.f;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      out[2 * j] = o[j][0] * inv;
-      out[2 * j + 1] = o[j][1] * inv;
+      out[2 * j] = (OP ? o[j][0] + o[j][2] : o[j][0]) * inv;
+      out[2 * j + 1] = (OP ? o[j][1] + o[j][3] : o[j][1]) * inv;
     }
   }
   for (int sp0 = 0; sp0 < a.n_splits; sp0 += 4) {

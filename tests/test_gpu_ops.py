@@ -392,3 +392,24 @@ def test_hybrid_attention_with_a_context_per_stream(tk, mask, dtype):
         wide = lambda t: t.expand(B, H, Nc, Dh)
         want, _ = ref_attention(q, torch.cat([wide(k), kb], 2), torch.cat([wide(v), vb], 2), full)
         assert float((got - want).abs().max() / want.abs().max()) <= tol
+
+
+def test_hybrid_attention_masked_bf16_keeps_the_numerators_at_fp32(tk):
+    """Private keys in pairs of opposite values and all but equal scores: the result is the difference of their
+    softmax numerators, 3.5e-4 of each, so their own accuracy shows through the bf16 result."""
+    B, H, Nb, Dh = 4, 2, 40, 32
+    g = torch.Generator(device="cuda").manual_seed(2)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g).bfloat16()
+    q, kb, vb = r(B, H, 1, Dh), r(B, H, Nb, Dh) / 2, r(B, H, Nb, Dh)
+    q[..., 31], q[..., 30] = 2.0 ** -6, 8.0
+    kb[:, :, 1::2], vb[:, :, 1::2] = kb[:, :, ::2], -vb[:, :, ::2]
+    kb[..., 30], kb[:, :, ::2, 31], kb[:, :, 1::2, 31] = 0.0, 0.0, 0.125
+    k, v = torch.zeros(H, 3, Dh, device="cuda").bfloat16(), r(H, 3, Dh)
+    k[..., 30] = -64.0                                           # the context weighs exp(-90)
+    mask = (torch.arange(Nb, device="cuda") // 2 % 3 != 0).view(1, 1, 1, Nb)
+    got = tk.hybrid_attention(q, k, v, kb, vb, buf_mask=mask).double()
+    s = (q.double() @ kb.double().transpose(-1, -2) * Dh ** -0.5).masked_fill(~mask, float("-inf"))
+    want = torch.softmax(s, -1) @ vb.double()
+    # bf16 result: 2^-9 at most, 1.1e-3 rms; numerators good to 2^-22 (the exponential): 2^-22 / 3.5e-4 = 7e-4.
+    # Numerators of 16 bits: 2^-17 / 3.5e-4 / sqrt(3) = 1.3e-2
+    assert float((got - want).norm() / want.norm()) <= 2 ** -8
