@@ -184,7 +184,8 @@ __device__ __forceinline__ float ex2_approx(float x) {
 // exponentials per clock and SM and is what bounds this kernel at head_dim 32): round x to the nearest
 // integer n with the 1.5 * 2^23 trick, a cubic for 2^f on f = x - n in [-0.5, 0.5] (relative error
 // 7.5e-5, far below the bf16 rounding of P), and n added into the exponent field.  x is clamped at
-// -125 (the result is then ~2e-38, i.e. nothing); x stays below ~2^4 here (lazy maximum).
+// -125 (the result is then ~2e-38, i.e. nothing); x stays below ~2^4 in the two-pass form (lazy maximum), the one-pass
+// form clamps it at 126.
 #ifndef ARTAB_POLY_EXP_OF_8
 #define ARTAB_POLY_EXP_OF_8 2   // of every 8 score pairs this many take the FMA-pipe exponential (measured best in both forms of the tile; one-pass, 8192 rows x 16384 keys: 2 -> 242 us, 1 -> 250, 3 -> 255, 0 -> 266)
 #endif
@@ -337,8 +338,9 @@ __device__ __forceinline__ bool softmax_tile(Smem* sm, uint32_t t_row, int wg, i
 // The same tile in ONE pass: exponentials against the reference the first tile left, whatever this tile's
 // maximum is.  No maximum pass, no exchange between the warpgroups, no rescale: the scores are read once.
 // That is exact in the reference (O / l and m + log2(l) do not depend on it) as long as nothing overflows:
-// the numerators may grow to kOnePassMax, and a row that passes that shows in its sum, upon which the CTA
-// walks its keys again with the two-pass form.  Two passes per tile -> one, 6 heads: 4096 rows x 8192 keys
+// the numerators may grow to kOnePassMax, and a row that passes that shows in its sum, an accumulator that
+// overflowed (numerators times a large V) in its value, upon which the CTA walks its keys again with the
+// two-pass form.  Two passes per tile -> one, 6 heads: 4096 rows x 8192 keys
 // 79.5 -> 69.5 us, 8192 x 16384 285 -> 242 us (2.83 -> 3.33e12 exponentials per second), 64 contexts of 2048
 // rows attending to themselves 595 -> 515 us.  Measured beside it and dropped: P and P . V in two chunks with
 // barriers of their own (261 us at 8192 x 16384), fewer reads of the clock in the waits (no change).
@@ -597,71 +599,77 @@ ctx_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     float m = -INFINITY, l = 0.f;
     uint32_t r[32];
     bool ok = true;
-    // On an abort the loop still runs every iteration (waits return at once, results are void):
+    // On an abort the loops still run every iteration (waits return at once, results are void):
     // both warpgroups must execute the same number of bar.sync instructions.
-    int last = nt - 1;   // number of the last tile walked
-    for (int i = 0; i <= last; ++i) {
-      const int j = i < nt ? i : i - nt;
-      ok = mbar_wait(&sm->s_full, i & 1, abort_flag) && ok;
-      tc_fence_after();
-      const int n_valid = p.n_ctx - (tile_begin + j) * BN;
-      if (j == 0 || i >= nt) {
-        if (n_valid >= BN)
-          ok = softmax_tile<false, NATURAL>(sm, t_row, wg, row, i & 1, sc, BN, m, l, j == 0, abort_flag) && ok;
-        else
-          ok = softmax_tile<true, NATURAL>(sm, t_row, wg, row, i & 1, sc, n_valid, m, l, j == 0, abort_flag) && ok;
-      } else {
-        if (n_valid >= BN)
-          ok = softmax_tile_one_pass<false>(sm, t_row, wg, (i & 1) ^ 1, sc, BN, m, l, abort_flag) && ok;
-        else
-          ok = softmax_tile_one_pass<true>(sm, t_row, wg, (i & 1) ^ 1, sc, n_valid, m, l, abort_flag) && ok;
+#pragma unroll 1
+    for (int i0 = 0;; i0 = nt) {   // first walk over the keys, second one
+#pragma unroll 1
+      for (int j = 0; j < nt; ++j) {
+        const int i = i0 + j;
+        ok = mbar_wait(&sm->s_full, i & 1, abort_flag) && ok;
+        tc_fence_after();
+        const int n_valid = p.n_ctx - (tile_begin + j) * BN;
+        if (j == 0 || i0) {
+          if (n_valid >= BN)
+            ok = softmax_tile<false, NATURAL>(sm, t_row, wg, row, i & 1, sc, BN, m, l, j == 0, abort_flag) && ok;
+          else
+            ok = softmax_tile<true, NATURAL>(sm, t_row, wg, row, i & 1, sc, n_valid, m, l, j == 0, abort_flag) && ok;
+        } else {
+          if (n_valid >= BN)
+            ok = softmax_tile_one_pass<false>(sm, t_row, wg, (i & 1) ^ 1, sc, BN, m, l, abort_flag) && ok;
+          else
+            ok = softmax_tile_one_pass<true>(sm, t_row, wg, (i & 1) ^ 1, sc, n_valid, m, l, abort_flag) && ok;
+        }
+        tmem_wait_st();
+        tc_fence_before();
+        mbar_arrive(&sm->p_full);
       }
-      tmem_wait_st();
-      tc_fence_before();
-      mbar_arrive(&sm->p_full);
-      if (i == nt - 1 && nt > 1) {
-        if (!(l < kOnePassMax)) sm->redo = 1;
+      if (wg == 1) sm->xsum[row] = l;
+      bool over = !(l < kOnePassMax);
+      asm volatile("bar.sync 2, 256;" ::: "memory");
+      ok = mbar_wait(&sm->o_full, (i0 + nt - 1) & 1, abort_flag) && ok;  // the last P . V is done
+      tc_fence_after();
+      if (nt > 1 && i0 == 0) {   // one-pass walk: repeat it with the two-pass form where something overflowed
+        if (wg == 0) {           // the accumulator, too: l is finite up to 2^100 per row, l times V need not be
+          tmem_ld32(t_row + kColO, r);
+          tmem_wait_ld();
+#pragma unroll
+          for (int d = 0; d < DH; ++d) over = over || !(fabsf(__uint_as_float(r[d])) <= 3.0e38f);
+        }
+        if (over) sm->redo = 1;
         asm volatile("bar.sync 2, 256;" ::: "memory");   // never times out: both warpgroups take the same decision
         const int redo = *(volatile int*)&sm->redo;
         mbar_arrive(&sm->verdict);
         if (redo) {
-          last = 2 * nt - 1;
           m = -INFINITY;
           l = 0.f;
-          ok = mbar_wait(&sm->o_full, i & 1, abort_flag) && ok;  // the last P . V has read P
-          tc_fence_after();
+          continue;
         }
       }
-    }
-    if (wg == 1) sm->xsum[row] = l;
-    asm volatile("bar.sync 2, 256;" ::: "memory");
-    if (wg == 0) {
+      if (wg == 1) break;
       l += sm->xsum[row];
-      if (ok) ok = mbar_wait(&sm->o_full, last & 1, abort_flag);
-      if (ok) {
-        tc_fence_after();
-        float o[DH];
-        tmem_ld32(t_row + kColO, r);          // P . V_hi
+      float o[DH];
+      tmem_ld32(t_row + kColO, r);          // P . V_hi
+      tmem_wait_ld();
+#pragma unroll
+      for (int d = 0; d < DH; ++d) o[d] = __uint_as_float(r[d]);
+      if constexpr (!NATURAL) {
+        tmem_ld32(t_row + kColO + 32, r);     // P . V_lo
         tmem_wait_ld();
 #pragma unroll
-        for (int d = 0; d < DH; ++d) o[d] = __uint_as_float(r[d]);
-        if constexpr (!NATURAL) {
-          tmem_ld32(t_row + kColO + 32, r);     // P . V_lo
-          tmem_wait_ld();
-#pragma unroll
-          for (int d = 0; d < DH; ++d) o[d] += __uint_as_float(r[d]);
-        }
-        if (row_valid) {
-          const float inv = 1.0f / l;
-#pragma unroll
-          for (int d = 0; d < DH; d += 4) {
-            float* dst = p.out + (p.out_lane_major ? lane_major_index(group_row0 + m0 + row, h * DH + d, p.n_heads * DH)
-                                                   : out_row * DH + d);
-            *reinterpret_cast<float4*>(dst) = make_float4(o[d] * inv, o[d + 1] * inv, o[d + 2] * inv, o[d + 3] * inv);
-          }
-          p.lse[out_row] = (m + log2f(l)) * kLn2;
-        }
+        for (int d = 0; d < DH; ++d) o[d] += __uint_as_float(r[d]);
       }
+      if (ok && row_valid) {
+        const float inv = 1.0f / l;
+#pragma unroll
+        for (int d = 0; d < DH; d += 4) {
+          float* dst = p.out + (p.out_lane_major ? lane_major_index(group_row0 + m0 + row, h * DH + d, p.n_heads * DH)
+                                                 : out_row * DH + d);
+          *reinterpret_cast<float4*>(dst) = make_float4(o[d] * inv, o[d + 1] * inv, o[d + 2] * inv, o[d + 3] * inv);
+        }
+        p.lse[out_row] = (m + log2f(l)) * kLn2;
+      }
+      break;
     }
   }
 

@@ -413,3 +413,23 @@ def test_hybrid_attention_masked_bf16_keeps_the_numerators_at_fp32(tk):
     # bf16 result: 2^-9 at most, 1.1e-3 rms; numerators good to 2^-22 (the exponential): 2^-22 / 3.5e-4 = 7e-4.
     # Numerators of 16 bits: 2^-17 / 3.5e-4 / sqrt(3) = 1.3e-2
     assert float((got - want).norm() / want.norm()) <= 2 ** -8
+
+
+@pytest.mark.parametrize("Nc", [200, 1000])
+@pytest.mark.parametrize("packed", [True, False])
+def test_large_values_behind_scores_far_above_the_first_key_tile(tk, packed, Nc):
+    """Scores of the later keys 52 nats (2^75) above the first tile's, V of 2^56: the softmax sums stay finite where
+    sums times V do not, and the result, about one V, has to be finite as well.  Packed and caller's own K / V."""
+    rows, H, Dh = 70, 2, 32
+    g = torch.Generator(device="cuda").manual_seed(4)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    q, k, v = r(rows, H, 1, Dh), r(H, Nc, Dh), r(H, Nc, Dh) * 2.0 ** 56
+    q[..., 0], k[..., 0] = 8.0, 0.0
+    k[:, 130:, 0] = 36.75
+    q, k, v = q.bfloat16(), k.bfloat16(), v.bfloat16()
+    kb, vb = torch.zeros(rows, H, 1, Dh, device="cuda").bfloat16(), torch.zeros(rows, H, 1, Dh, device="cuda").bfloat16()
+    got = (tk.triton_context_attention(q, k, v)[0] if packed else tk.hybrid_attention(q, k, v, kb, vb)).double()
+    s = q.double() @ k.double().transpose(-1, -2) * Dh ** -0.5
+    want = torch.softmax(s, -1) @ v.double()
+    assert bool(got.isfinite().all())
+    assert float((got - want).norm() / want.norm()) <= 1e-2      # numerators and results rounded to 8 bits
