@@ -625,51 +625,48 @@ ctx_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         mbar_arrive(&sm->p_full);
       }
       if (wg == 1) sm->xsum[row] = l;
-      bool over = !(l < kOnePassMax);
+      const bool one_pass = nt > 1 && i0 == 0;
+      if (one_pass && !(l < kOnePassMax)) sm->redo = 1;
       asm volatile("bar.sync 2, 256;" ::: "memory");
       ok = mbar_wait(&sm->o_full, (i0 + nt - 1) & 1, abort_flag) && ok;  // the last P . V is done
       tc_fence_after();
-      if (nt > 1 && i0 == 0) {   // one-pass walk: repeat it with the two-pass form where something overflowed
-        if (wg == 0) {           // the accumulator, too: l is finite up to 2^100 per row, l times V need not be
-          tmem_ld32(t_row + kColO, r);
-          tmem_wait_ld();
-#pragma unroll
-          for (int d = 0; d < DH; ++d) over = over || !(fabsf(__uint_as_float(r[d])) <= 3.0e38f);
-        }
-        if (over) sm->redo = 1;
-        asm volatile("bar.sync 2, 256;" ::: "memory");   // never times out: both warpgroups take the same decision
-        const int redo = *(volatile int*)&sm->redo;
-        mbar_arrive(&sm->verdict);
-        if (redo) {
-          m = -INFINITY;
-          l = 0.f;
-          continue;
-        }
-      }
-      if (wg == 1) break;
-      l += sm->xsum[row];
-      float o[DH];
-      tmem_ld32(t_row + kColO, r);          // P . V_hi
-      tmem_wait_ld();
-#pragma unroll
-      for (int d = 0; d < DH; ++d) o[d] = __uint_as_float(r[d]);
-      if constexpr (!NATURAL) {
-        tmem_ld32(t_row + kColO + 32, r);     // P . V_lo
+      if (wg == 0) {
+        l += sm->xsum[row];
+        float o[DH];
+        tmem_ld32(t_row + kColO, r);          // P . V_hi
         tmem_wait_ld();
 #pragma unroll
-        for (int d = 0; d < DH; ++d) o[d] += __uint_as_float(r[d]);
-      }
-      if (ok && row_valid) {
-        const float inv = 1.0f / l;
+        for (int d = 0; d < DH; ++d) o[d] = __uint_as_float(r[d]);
+        if constexpr (!NATURAL) {
+          tmem_ld32(t_row + kColO + 32, r);     // P . V_lo
+          tmem_wait_ld();
 #pragma unroll
-        for (int d = 0; d < DH; d += 4) {
-          float* dst = p.out + (p.out_lane_major ? lane_major_index(group_row0 + m0 + row, h * DH + d, p.n_heads * DH)
-                                                 : out_row * DH + d);
-          *reinterpret_cast<float4*>(dst) = make_float4(o[d] * inv, o[d + 1] * inv, o[d + 2] * inv, o[d + 3] * inv);
+          for (int d = 0; d < DH; ++d) o[d] += __uint_as_float(r[d]);
         }
-        p.lse[out_row] = (m + log2f(l)) * kLn2;
+        if (one_pass) {   // l is finite up to 2^100 per row, l times V need not be
+          bool over = false;
+#pragma unroll
+          for (int d = 0; d < DH; ++d) over = over || !(fabsf(o[d]) <= 3.0e38f);
+          if (over) sm->redo = 1;
+        }
+        if (ok && row_valid) {   // a second walk writes them again
+          const float inv = 1.0f / l;
+#pragma unroll
+          for (int d = 0; d < DH; d += 4) {
+            float* dst = p.out + (p.out_lane_major ? lane_major_index(group_row0 + m0 + row, h * DH + d, p.n_heads * DH)
+                                                   : out_row * DH + d);
+            *reinterpret_cast<float4*>(dst) = make_float4(o[d] * inv, o[d + 1] * inv, o[d + 2] * inv, o[d + 3] * inv);
+          }
+          p.lse[out_row] = (m + log2f(l)) * kLn2;
+        }
       }
-      break;
+      if (!one_pass) break;
+      asm volatile("bar.sync 2, 256;" ::: "memory");   // never times out: both warpgroups take the same decision
+      const int redo = *(volatile int*)&sm->redo;
+      mbar_arrive(&sm->verdict);
+      if (!redo) break;
+      m = -INFINITY;
+      l = 0.f;
     }
   }
 
