@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
+
 #include "artab.h"
 
 namespace artab {
@@ -104,9 +106,11 @@ struct PlainLaunchScope {
 };
 
 // Largest dynamic shared-memory size a kernel has been configured for, per device: the opt-in is a
-// per-device attribute, so a process that uses several GPUs repeats it on each.
+// per-device attribute, so a process that uses several GPUs repeats it on each.  The attribute is set, not
+// raised: a kernel has ONE of these, whoever configures it (launch, occupancy query) and from any thread.
 constexpr int kMaxDevices = 64;
 struct SmemConfig {
+  std::mutex lock;
   size_t bytes[kMaxDevices] = {};
   // several_per_sm: the kernel is meant to have more than one CTA resident per SM, so it also asks
   // for the largest shared-memory carve-out (the default heuristic may pick one that fits a single CTA)
@@ -116,6 +120,7 @@ struct SmemConfig {
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     const bool tracked = dev >= 0 && dev < kMaxDevices;
+    std::lock_guard<std::mutex> guard(lock);
     if (tracked && smem <= bytes[dev]) return cudaSuccess;
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess && several_per_sm)

@@ -516,15 +516,24 @@ __global__ void __launch_bounds__(kThreads, 1) dense_mma_kernel(const __grid_con
   }
 }
 
+template <int D>
+SmemConfig& smem_config() {
+  static SmemConfig c;
+  return c;
+}
+
+constexpr int kMaxDff = 1024;   // of the weight tiles this chain takes (dense_tc_applicable)
+
 // rows of the clusters that fit the GPU at once
 template <int D>
-int rows_at_once(size_t smem) {
-  static thread_local int rows[kMaxDevices];
+int rows_at_once(int d_ff) {
+  static thread_local int cached[kMaxDevices][kMaxDff / 128 + 1];
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
-  if (rows[dev]) return rows[dev];
-  static SmemConfig configured;
-  if (configured.ensure(dense_mma_kernel<D>, smem) != cudaSuccess) return 0;
+  if (d_ff > kMaxDff || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
+  int& rows = cached[dev][d_ff / 128];
+  if (rows) return rows;
+  const size_t smem = plan_of(D, d_ff / kC).total;
+  if (smem_config<D>().ensure(dense_mma_kernel<D>, smem) != cudaSuccess) return 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(kC);
   cfg.blockDim = dim3(kThreads);
@@ -541,14 +550,13 @@ int rows_at_once(size_t smem) {
     cudaGetLastError();
     return 0;
   }
-  return rows[dev] = n * kRows;
+  return rows = n * kRows;
 }
 
 template <int D>
 int launch_d(const DenseArgs& a, cudaStream_t s) {
   const size_t smem = plan_of(D, a.Dff / kC).total;
-  static SmemConfig configured;
-  cudaError_t e = configured.ensure(dense_mma_kernel<D>, smem);
+  cudaError_t e = smem_config<D>().ensure(dense_mma_kernel<D>, smem);
   prof_begin(PROF_DENSE, s);
   if (e == cudaSuccess)
     e = launch_dependent_cluster(dense_mma_kernel<D>, dim3((a.rows + kRows - 1) / kRows * kC), dim3(kThreads), smem, s, kC, a);
@@ -564,8 +572,7 @@ int launch_d(const DenseArgs& a, cudaStream_t s) {
 bool dense_mma_applicable(const DenseArgs& a) {
   if (!a.lane_major || !(a.do_pre || (a.do_post && a.do_head)) || a.x_out || a.z_out || !dense_tc_applicable(a)) return false;
   if ((a.do_post && !a.post_w.mma_post) || (a.do_pre && !a.pre_w.mma_pre) || (a.do_head && !a.mma_head)) return false;
-  const size_t smem = plan_of(a.D, a.Dff / kC).total;
-  const int most = a.D == 64 ? rows_at_once<64>(smem) : a.D == 128 ? rows_at_once<128>(smem) : rows_at_once<192>(smem);
+  const int most = a.D == 64 ? rows_at_once<64>(a.Dff) : a.D == 128 ? rows_at_once<128>(a.Dff) : rows_at_once<192>(a.Dff);
   return a.rows <= most;
 }
 

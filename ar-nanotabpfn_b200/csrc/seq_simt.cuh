@@ -801,9 +801,14 @@ __global__ void __launch_bounds__(kT + 32, 1) seq_simt_kernel(const __grid_const
 }
 
 template <typename CT, int DH, int R, bool SHARED>
+SmemConfig& smem_config() {
+  static SmemConfig c;
+  return c;
+}
+
+template <typename CT, int DH, int R, bool SHARED>
 int launch_seq_variant(const SeqArgs& a, const SeqPlan& p, cudaStream_t s) {
-  static SmemConfig configured;
-  cudaError_t e = configured.ensure(seq_simt_kernel<CT, DH, R, SHARED>, p.smem);
+  cudaError_t e = smem_config<CT, DH, R, SHARED>().ensure(seq_simt_kernel<CT, DH, R, SHARED>, p.smem);
   if (e == cudaSuccess)
     e = launch_dependent_cluster(seq_simt_kernel<CT, DH, R, SHARED>, dim3(p.grid), dim3(kT + 32), p.smem, s, (unsigned)p.C, a);
   ARTAB_REQUIRE(e == cudaSuccess, ARTAB_ELAUNCH, "seq_simt_kernel: launch refused: %s", cudaGetErrorString(e));
@@ -831,8 +836,7 @@ int launch_seq_dh(const SeqArgs& a, const SeqPlan& p, cudaStream_t s) {
 // clusters of C CTAs that fit the GPU at once (every variant takes a whole SM per CTA)
 template <typename CT>
 int seq_max_clusters(int C, size_t smem) {
-  static SmemConfig configured;
-  if (configured.ensure(seq_simt_kernel<CT, 32, 8, true>, smem) != cudaSuccess) return 0;
+  if (smem_config<CT, 32, 8, true>().ensure(seq_simt_kernel<CT, 32, 8, true>, smem) != cudaSuccess) return 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(C);
   cfg.blockDim = dim3(kT + 32);
