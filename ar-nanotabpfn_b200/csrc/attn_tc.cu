@@ -476,6 +476,7 @@ ctx_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  int issued = 0;   // K / V tiles the producer thread (0) has asked for
   const uint32_t tmem = sm->tmem_base;
   volatile int* abort_flag = &sm->ctl.abort_flag;
   if (warp != 0) {  // the producer waits after its early K/V prefetch
@@ -489,7 +490,6 @@ ctx_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     if (lane == 0) {
       const int krow0 = (g * p.n_heads + h) * p.n_ctx_pad;
       const int vrow0 = (g * p.n_heads + h) * 2 * DH;
-      int issued = 0;
       auto load_kv = [&](int st, int j) {
         const int key0 = (tile_begin + j) * BN;
         if constexpr (NATURAL) {  // rows past a head's last key read as zero
@@ -519,18 +519,6 @@ ctx_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       };
       walk(nt);
       if (nt > 1 && mbar_wait(&sm->verdict, 0, abort_flag) && *(volatile int*)&sm->redo) walk(2 * nt);
-      if (*abort_flag) {  // drain our own copies before the CTA may exit
-        {
-          const long long t0 = clock64();
-          while (!mbar_try(&sm->q_full, 0) && clock64() - t0 < p.wait_cycles) {
-          }
-        }
-        for (int j = max(0, issued - NSTAGE); j < issued; ++j) {
-          const long long t0 = clock64();
-          while (!mbar_try(&sm->kv_full[j % NSTAGE], (j / NSTAGE) & 1) && clock64() - t0 < p.wait_cycles) {
-          }
-        }
-      }
     }
   } else if (warp == 1) {
     // ------------------------------- MMA issuer -------------------------------
@@ -676,7 +664,16 @@ ctx_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
   }
-  if (threadIdx.x == 0 && sm->ctl.abort_flag && p.status) atomicExch(p.status, 1);
+  if (threadIdx.x == 0 && sm->ctl.abort_flag) {   // the producer's own copies have to land before the CTA may exit
+    if (p.status) atomicExch(p.status, 1);
+    auto landed = [](uint64_t* b, int parity) {
+      const long long t0 = clock64();
+      while (!mbar_try(b, parity) && clock64() - t0 < kWaitCycles) {
+      }
+    };
+    landed(&sm->q_full, 0);
+    for (int j = max(0, issued - NSTAGE); j < issued; ++j) landed(&sm->kv_full[j % NSTAGE], (j / NSTAGE) & 1);
+  }
   if (p.cta_status) {
     if (threadIdx.x == 0) p.cta_status[(blockIdx.z * gridDim.y + h) * gridDim.x + blockIdx.x] = sm->ctl.abort_flag ? 1 : 0;
     if (sm->ctl.abort_flag && row_valid) p.lse[out_row] = INFINITY;

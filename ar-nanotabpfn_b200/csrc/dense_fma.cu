@@ -10,6 +10,7 @@
 // Q, K, V | out-projection, then for every D-wide chunk of the hidden layer W1 and W2, whose products
 // accumulate in registers, so the hidden layer never exists as a whole.  A producer warp streams 32-row slabs
 // of the panels through a ring of bulk copies.
+#include "cluster.cuh"
 #include "dense.cuh"
 #include "head.cuh"
 #include "kv_scatter.cuh"
@@ -37,30 +38,21 @@ struct Bars {
   int abort_flag;
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ bool mbar_try(uint64_t* b, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(b)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// bounded; false once the CTA is aborting
-__device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity, volatile int* abort_flag) {
-  if (mbar_try(b, parity)) return true;
+__device__ __noinline__ void wait_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   const long long t0 = clock64();
   for (;;) {
-    if (*abort_flag) return false;
-    if (mbar_try(b, parity)) return true;
+    if (*abort_flag) return;   // first: after an abort no wait may block again
     if (clock64() - t0 > kWaitCycles) {
       *abort_flag = 1;
-      return false;
+      return;
     }
+    if (mbar_try(bar, parity)) return;
   }
+}
+// bounded; on return the phase is over or the CTA is aborting
+__device__ __forceinline__ void mbar_wait(uint64_t* b, uint32_t parity, int* abort_flag) {
+  const uint32_t bar = smem_u32(b);
+  if (!mbar_test(bar, parity)) wait_slow(bar, parity, abort_flag);
 }
 template <int T>
 __device__ __forceinline__ void sync_compute() { asm volatile("bar.sync 1, %0;" ::"n"(T) : "memory"); }
@@ -187,13 +179,14 @@ __global__ void __launch_bounds__(Shape<D>::T + 32, D == 64 ? 2 : 1) dense_fma_k
 
   if (tid >= S::T) {
     // ------------------------------ producer warp ------------------------------
+    int issued = 0;
     if (tid == S::T) {
-      int issued = 0;
       auto stream = [&](const float* w, int panels) {
 #pragma unroll 1
         for (int i = 0; i < panels * (D / 32); ++i, w += S::SLAB) {
           const int slot = issued % kSlots;
-          if (issued >= kSlots && !mbar_wait(&bars->empty[slot], ((issued / kSlots) + 1) & 1, &bars->abort_flag)) return;
+          if (issued >= kSlots) mbar_wait(&bars->empty[slot], ((issued / kSlots) + 1) & 1, &bars->abort_flag);
+          if (*(volatile int*)&bars->abort_flag) return;
           asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&bars->full[slot])),
                        "r"(S::SLAB * 4)
                        : "memory");
@@ -207,11 +200,12 @@ __global__ void __launch_bounds__(Shape<D>::T + 32, D == 64 ? 2 : 1) dense_fma_k
       if (a.do_post) stream(a.post_w.fma_post, 1 + 2 * n_hidden);
       if (a.do_head) stream(a.fma_head, 2 * n_hidden);
       else if (a.do_pre) stream(a.pre_w.fma_pre, 4);
-      if (bars->abort_flag) {  // let the copies in flight land before the CTA may exit
-        for (int i = max(0, issued - kSlots); i < issued; ++i) {
-          const long long t0 = clock64();
-          while (!mbar_try(&bars->full[i % kSlots], (i / kSlots) & 1) && clock64() - t0 < kWaitCycles) {
-          }
+    }
+    __syncthreads();   // the compute threads are done, or have given up: then the copies in flight land before the CTA may exit
+    if (tid == S::T && bars->abort_flag) {
+      for (int i = max(0, issued - kSlots); i < issued; ++i) {
+        const long long t0 = clock64();
+        while (!mbar_try(smem_u32(&bars->full[i % kSlots]), (i / kSlots) & 1) && clock64() - t0 < kWaitCycles) {
         }
       }
     }
@@ -304,6 +298,7 @@ __global__ void __launch_bounds__(Shape<D>::T + 32, D == 64 ? 2 : 1) dense_fma_k
       }
     }
   }
+  __syncthreads();
   if (tid == 0 && bars->abort_flag && a.status) atomicExch(a.status, 5);
 }
 

@@ -35,6 +35,7 @@ namespace {
 
 constexpr int kWarps = kSeqWarps;      // compute warps
 constexpr int kT = kSeqThreads;        // compute threads
+constexpr long long kDrainCycles = 2000000000LL;  // about one second: for copies in flight after an abort
 constexpr int kP = kSeqPitch;          // floats between the rows of every activation array
 
 extern __shared__ __align__(1024) uint8_t g_seq_smem[];
@@ -50,6 +51,19 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
 }
 __device__ __forceinline__ float gelu_erf(float v) { return 0.5f * v * (1.0f + erff(v * 0.70710678118654752f)); }
 __device__ __forceinline__ void sync_compute() { asm volatile("bar.sync 1, %0;" ::"n"(kT) : "memory"); }
+// the same, and whether `v` is non-zero in any compute thread: one answer for all of them
+__device__ __forceinline__ bool sync_compute_any(int v) {
+  int any;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.s32 q, %1, 0;\n\t"
+      "bar.red.or.pred p, 1, %2, q;\n\t"
+      "selp.s32 %0, 1, 0, p;\n\t}"
+      : "=r"(any)
+      : "r"(v), "n"(kT)
+      : "memory");
+  return any != 0;
+}
 
 // mbarriers (full / empty per ring slot, one per exchange) and what a bounded wait needs, at the start of
 // shared memory: a wait site hands over nothing but the barrier.
@@ -68,11 +82,11 @@ __device__ __noinline__ void wait_slow(uint32_t bar, uint32_t parity) {
   const long long t0 = clock64();
   for (;;) {
     if (b->abort_flag) return;  // first: after an abort no wait may block again
-    if (mbar_try(bar, parity)) return;
     if (clock64() - t0 > b->limit) {
       b->abort_flag = 1;
       return;
     }
+    if (mbar_try(bar, parity)) return;
   }
 }
 // Bounded wait.  The data behind every barrier of this kernel (bulk copies, st.async of a peer) land in this
@@ -361,11 +375,11 @@ __global__ void __launch_bounds__(kT + 32, 1) seq_simt_kernel(const __grid_const
   dep_trigger();
   volatile int* abort_flag = &bars->abort_flag;
 
+  int slot = 0, filled = 0;   // producer thread: next ring slot, slots ever filled
+  uint32_t phase = 1;         // empty barriers: the first round passes at once
   if (warp == kWarps) {
     // ------------------------------- producer -------------------------------
     if (lane == 0) {
-      int slot = 0, filled = 0;
-      uint32_t phase = 1;  // empty barriers: the first round passes at once
       auto put = [&](const void* src, uint32_t bytes) {
         if (*abort_flag) return;
         wait_bar(smem_u32(&bars->empty[slot]), phase);
@@ -420,17 +434,6 @@ __global__ void __launch_bounds__(kT + 32, 1) seq_simt_kernel(const __grid_const
           }
         }
       }
-      // after a wait that gave up: let the copies in flight land before the CTA may exit
-      if (*abort_flag) {
-#pragma unroll 1
-        for (int i = 0; i < n_slots; ++i) {
-          if (!((filled >> i) & 1)) continue;
-          const uint32_t par = i < slot ? phase ^ 1 : phase;   // phase in which slot i was last filled
-          const long long t0 = clock64();
-          while (!mbar_try(smem_u32(&bars->full[i]), par) && clock64() - t0 < a.wait_cycles) {
-          }
-        }
-      }
     }
     __syncwarp();
   } else {
@@ -482,6 +485,7 @@ __global__ void __launch_bounds__(kT + 32, 1) seq_simt_kernel(const __grid_const
     }
     sync_compute();
 
+    bool dead = false;
 #pragma unroll 1
     for (int t = a.t0; t < a.t1; ++t) {
       const int len = t;               // private keys visible in this step (the buffer token's own among them)
@@ -682,7 +686,11 @@ __global__ void __launch_bounds__(kT + 32, 1) seq_simt_kernel(const __grid_const
           const uint32_t par = xparity(0);
           if (warp == 0) wait_bar(xbar0, par);  // one warp polls, the others sleep at the barrier
         }
-        sync_compute();   // also: the scratch has been read, the projections may overwrite it
+        // Also: the scratch has been read, the projections may overwrite it.  And where a job ends whose waits gave
+        // up: until here every exchange barrier has been armed at most once since, so none is armed twice in a phase,
+        // and the peers, which get nothing more from here, give up in turn.
+        dead = sync_compute_any(*abort_flag);
+        if (dead) break;
         // ---- out-projection, MLP; the last layer has results for the target rows only ----
         auto post = [&](auto rows_const, auto ld_const, int off) {
           constexpr int RR = decltype(rows_const)::value, LD = decltype(ld_const)::value;
@@ -721,6 +729,7 @@ __global__ void __launch_bounds__(kT + 32, 1) seq_simt_kernel(const __grid_const
         SEQ_TL(16 * l + 12);
       }
 
+      if (dead) break;
       SEQ_TL(16 * L);
       // ---- mixture head on the target rows: every CTA ends up with all raw outputs ----
       layer_norm(z, kP, res + kP, 2 * kP, nullptr, 0, nullptr, S, D, vec + L * (7 * D + HS), vec + L * (7 * D + HS) + D, 0, 0);
@@ -789,15 +798,27 @@ __global__ void __launch_bounds__(kT + 32, 1) seq_simt_kernel(const __grid_const
     }
   }
 
-  // nobody leaves while another CTA could still write here; after an abort, stores may be in flight
+  // Nobody leaves while another CTA could still write here.  Without an abort every store has been waited for; after
+  // one the peers have issued their last when the barrier opens, and some may be in flight.
+  __syncthreads();
+  if (bars->abort_flag && warp == kWarps && lane == 0) {   // the copies in flight land first, too
+#pragma unroll 1
+    for (int i = 0; i < n_slots; ++i) {
+      if (!((filled >> i) & 1)) continue;
+      const uint32_t par = i < slot ? phase ^ 1 : phase;   // phase in which slot i was last filled
+      const long long t0 = clock64();
+      while (!mbar_try(smem_u32(&bars->full[i]), par) && clock64() - t0 < kDrainCycles) {
+      }
+    }
+  }
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (bars->abort_flag) {
     if (tid == 0 && a.status) atomicExch(a.status, 4);
     const long long t0 = clock64();
     while (clock64() - t0 < 100000) {
     }
   }
-  __syncthreads();
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 template <typename CT, int DH, int R, bool SHARED>

@@ -141,3 +141,59 @@ def test_predictor_raises_after_a_timed_out_call():
     # the error is reported once; the predictor then works again
     assert torch.equal(p.evaluate_joint_density(xc, yc, xt, yt), good)
     assert p.last_status() == 0
+
+
+def _network(precision, **cfg):
+    from ar_tabpfn import ARTabPFN
+    from ar_tabpfn.model import ARTabPFNPredictor
+    torch.manual_seed(2)
+    m = ARTabPFN(num_features=4, num_components=5, **cfg).eval()
+    with torch.no_grad():
+        for p in m.parameters():
+            p.copy_(p.bfloat16().float())
+    return ARTabPFNPredictor.from_trained_model(m.cuda(), backend="triton_shared_context", precision=precision)
+
+
+def _rows(B, Nc, Nt):
+    g = torch.Generator(device="cuda").manual_seed(6)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    return r(1, Nc, 4).expand(B, -1, -1), r(1, Nc).expand(B, -1), r(B, Nt, 4), r(B, Nt)
+
+
+@pytest.mark.parametrize("B,heads,Nc", [(1, 4, 40), (130, 4, 1100), (40, 8, 33), (9, 12, 70)])
+def test_whole_sequence_decode_gives_up_and_the_next_one_is_correct(B, heads, Nc):
+    """A limit of one cycle: the first wait for a copy or a peer that has not arrived yet ends the job in every CTA."""
+    import ctypes as C
+    from ar_tabpfn import _lib
+    lib = _lib.lib()
+    p = _network("fp32", d_model=192 if heads == 12 else 128, n_heads=heads, n_layers=3, d_ff=384 if heads == 12 else 256)
+    Nt = 7
+    xc, yc, xt, _ = _rows(B, Nc, Nt)
+    expo, normal = torch.rand(Nt, B, 5, device="cuda") + 0.1, torch.randn(Nt, B, device="cuda")
+    p.init_kv_cache(B, Nt, xc.device, torch.float32)
+    p.prefill_context(xc, yc)
+    pm, st = p._packed(p._device), p._state
+    need = int(lib.artab_sequence_workspace(pm.ref, C.byref(st)))
+    assert need > 0
+    ws, status = torch.empty(need, dtype=torch.uint8, device="cuda"), p._bufs["status"]
+
+    def decode():
+        samples, ld = torch.full((B, Nt), -7.0, device="cuda"), torch.empty(B, Nt, device="cuda")
+        comp = torch.empty(B, Nt, dtype=torch.int32, device="cuda")
+        st.buffer_len = 0
+        status.zero_()
+        _lib.check(lib.artab_decode_sequence(pm.ref, C.byref(st), _lib.ptr(xt), Nt * 4, 4, Nt, 0, Nt, _lib.ptr(samples),
+                                             _lib.ptr(expo), _lib.ptr(normal), _lib.ptr(ld), _lib.ptr(comp), _lib.ptr(ws),
+                                             need, _lib.stream_ptr()))
+        torch.cuda.synchronize()
+        return samples, int(status.item())
+    good, code = decode()
+    assert code == 0 and bool(good.isfinite().all()) and bool((good != -7.0).all())
+    try:
+        _lib.check(lib.artab_debug_set(_lib.DEBUG_WAIT_CYCLES, 1))
+        void, code = decode()
+    finally:
+        lib.artab_debug_set(_lib.DEBUG_WAIT_CYCLES, 0)
+    assert code == 4 and bool((void == -7.0).all())
+    again, code = decode()
+    assert code == 0 and torch.equal(again, good)
