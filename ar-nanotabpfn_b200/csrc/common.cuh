@@ -95,6 +95,7 @@ bool dependent_launch_enabled();
 // diagnostics set through artab_debug_set: limit of the bounded waits (0: the built-in second or so) and
 // the switch that makes the context kernel's waits run out (see artab.h)
 long long debug_wait_cycles();
+constexpr long long kDefaultWaitCycles = 2000000000LL;   // about one second
 int debug_drop_score_commits();
 
 // While one of these lives on the calling thread, launch_dependent* issue plain launches.

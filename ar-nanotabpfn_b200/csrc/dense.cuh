@@ -48,6 +48,7 @@ struct DenseArgs {
   float* ld_out;
   int32_t* comp_out;
   int32_t* status;     // device status word (bounded waits), may be null
+  long long wait_cycles;  // limit of the waits of dense_fma / dense_mma, set by their launches
   // tensor-core chain: scratch for the CTA-pair exchange, pair_slots slots of pair_slot_stride floats
   // (>= rows rounded up to 128, times D, each); null: one CTA per row tile
   float* pair_scratch;

@@ -20,7 +20,6 @@ namespace artab {
 namespace {
 
 constexpr int kSlots = 4;
-constexpr long long kWaitCycles = 2000000000LL;
 
 extern __shared__ __align__(128) uint8_t g_fma_smem[];
 
@@ -35,24 +34,25 @@ struct Shape {
 
 struct Bars {
   uint64_t full[kSlots], empty[kSlots];
+  long long limit;
   int abort_flag;
 };
 
-__device__ __noinline__ void wait_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+__device__ __noinline__ void wait_slow(uint32_t bar, uint32_t parity, volatile Bars* b) {
   const long long t0 = clock64();
   for (;;) {
-    if (*abort_flag) return;   // first: after an abort no wait may block again
-    if (clock64() - t0 > kWaitCycles) {
-      *abort_flag = 1;
+    if (b->abort_flag) return;   // first: after an abort no wait may block again
+    if (clock64() - t0 > b->limit) {
+      b->abort_flag = 1;
       return;
     }
     if (mbar_try(bar, parity)) return;
   }
 }
 // bounded; on return the phase is over or the CTA is aborting
-__device__ __forceinline__ void mbar_wait(uint64_t* b, uint32_t parity, int* abort_flag) {
+__device__ __forceinline__ void mbar_wait(uint64_t* b, uint32_t parity, Bars* bars) {
   const uint32_t bar = smem_u32(b);
-  if (!mbar_test(bar, parity)) wait_slow(bar, parity, abort_flag);
+  if (!mbar_test(bar, parity)) wait_slow(bar, parity, bars);
 }
 template <int T>
 __device__ __forceinline__ void sync_compute() { asm volatile("bar.sync 1, %0;" ::"n"(T) : "memory"); }
@@ -72,7 +72,7 @@ struct Chain {
 #pragma unroll 1
     for (int s = 0; s < D / 32; ++s, x += 32) {
       const int slot = used % kSlots;
-      mbar_wait(&bars->full[slot], (used / kSlots) & 1, &bars->abort_flag);
+      mbar_wait(&bars->full[slot], (used / kSlots) & 1, bars);
       const float4* w = reinterpret_cast<const float4*>(ring + slot * S::SLAB) + cg;
 #pragma unroll 1
       for (int k = 0; k < 8; ++k) {
@@ -173,6 +173,7 @@ __global__ void __launch_bounds__(Shape<D>::T + 32, D == 64 ? 2 : 1) dense_fma_k
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&bars->empty[i])), "r"(S::T / 32) : "memory");
     }
     bars->abort_flag = 0;
+    bars->limit = a.wait_cycles;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
@@ -185,7 +186,7 @@ __global__ void __launch_bounds__(Shape<D>::T + 32, D == 64 ? 2 : 1) dense_fma_k
 #pragma unroll 1
         for (int i = 0; i < panels * (D / 32); ++i, w += S::SLAB) {
           const int slot = issued % kSlots;
-          if (issued >= kSlots) mbar_wait(&bars->empty[slot], ((issued / kSlots) + 1) & 1, &bars->abort_flag);
+          if (issued >= kSlots) mbar_wait(&bars->empty[slot], ((issued / kSlots) + 1) & 1, bars);
           if (*(volatile int*)&bars->abort_flag) return;
           asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&bars->full[slot])),
                        "r"(S::SLAB * 4)
@@ -205,7 +206,7 @@ __global__ void __launch_bounds__(Shape<D>::T + 32, D == 64 ? 2 : 1) dense_fma_k
     if (tid == S::T && bars->abort_flag) {
       for (int i = max(0, issued - kSlots); i < issued; ++i) {
         const long long t0 = clock64();
-        while (!mbar_try(smem_u32(&bars->full[i % kSlots]), (i / kSlots) & 1) && clock64() - t0 < kWaitCycles) {
+        while (!mbar_try(smem_u32(&bars->full[i % kSlots]), (i / kSlots) & 1) && clock64() - t0 < kDefaultWaitCycles) {
         }
       }
     }
@@ -303,7 +304,9 @@ __global__ void __launch_bounds__(Shape<D>::T + 32, D == 64 ? 2 : 1) dense_fma_k
 }
 
 template <typename T, int D, int TR>
-int launch_variant(const DenseArgs& a, cudaStream_t s) {
+int launch_variant(const DenseArgs& args, cudaStream_t s) {
+  DenseArgs a = args;
+  a.wait_cycles = debug_wait_cycles() > 0 ? debug_wait_cycles() : kDefaultWaitCycles;
   using S = Shape<D>;
   constexpr int R = S::RG * TR;
   const size_t smem = (size_t)(kSlots * S::SLAB + 2 * R * S::P) * sizeof(float) + sizeof(Bars);

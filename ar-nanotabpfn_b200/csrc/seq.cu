@@ -10,7 +10,6 @@ namespace artab {
 namespace {
 
 constexpr size_t kSmemMax = 227 * 1024;
-constexpr long long kWaitCycles = 2000000000LL;  // about one second
 constexpr int kMaxRowsPerCluster = 16;
 constexpr size_t kWorkspaceMax = (size_t)4 << 30;
 
@@ -229,7 +228,7 @@ int launch_seq(const artab_model* m, const artab_state* st, const SeqCall& c, cu
   a.logdens = c.logdens;
   a.comp = c.comp;
   a.status = st->status;
-  a.wait_cycles = debug_wait_cycles() > 0 ? debug_wait_cycles() : kWaitCycles;
+  a.wait_cycles = debug_wait_cycles() > 0 ? debug_wait_cycles() : kDefaultWaitCycles;
   a.scale_log2e = kLog2e / sqrtf((float)m->head_dim);
   prof_begin(PROF_DENSE, s);
   int rc;

@@ -35,7 +35,6 @@ namespace {
 
 constexpr int kWarps = kSeqWarps;      // compute warps
 constexpr int kT = kSeqThreads;        // compute threads
-constexpr long long kDrainCycles = 2000000000LL;  // about one second: for copies in flight after an abort
 constexpr int kP = kSeqPitch;          // floats between the rows of every activation array
 
 extern __shared__ __align__(1024) uint8_t g_seq_smem[];
@@ -807,7 +806,7 @@ __global__ void __launch_bounds__(kT + 32, 1) seq_simt_kernel(const __grid_const
       if (!((filled >> i) & 1)) continue;
       const uint32_t par = i < slot ? phase ^ 1 : phase;   // phase in which slot i was last filled
       const long long t0 = clock64();
-      while (!mbar_try(smem_u32(&bars->full[i]), par) && clock64() - t0 < kDrainCycles) {
+      while (!mbar_try(smem_u32(&bars->full[i]), par) && clock64() - t0 < kDefaultWaitCycles) {
       }
     }
   }

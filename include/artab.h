@@ -397,10 +397,12 @@ ARTAB_API int artab_profile_read(double* ms_per_kind, int64_t* launches_per_kind
 ARTAB_API void artab_set_dependent_launch(int on);
 
 /* Diagnostics of the bounded device-side waits (process-wide, off by default; no counterpart in
- * the reference).  Every mbarrier wait inside the tensor-core kernels gives up after a limit, the
- * CTA then writes nothing more, frees what it holds, sets the status word and returns.
- *   ARTAB_DEBUG_WAIT_CYCLES        value = limit in SM clock cycles for the context contraction's waits
- *                                  (0 restores the built-in limit of about one second)
+ * the reference).  Every mbarrier wait inside the kernels gives up after a limit, the CTA then waits for
+ * what it has in flight, frees what it holds, sets the status word and returns; results of the call are void.
+ *   ARTAB_DEBUG_WAIT_CYCLES        value = limit in SM clock cycles for the waits of the context contraction, the
+ *                                  whole-sequence decode and the register-tiled chain (0 restores the
+ *                                  built-in limit of about one second; the other dense chains always have
+ *                                  that, except that the few-row chain gives up at once with a limit of 1)
  *   ARTAB_DEBUG_DROP_SCORE_COMMITS value != 0: the context contraction's MMA thread never signals
  *                                  "scores ready", so its softmax threads' waits run out.  This is how
  *                                  the tests exercise the give-up path without faulting anything:

@@ -160,6 +160,36 @@ def _rows(B, Nc, Nt):
     return r(1, Nc, 4).expand(B, -1, -1), r(1, Nc).expand(B, -1), r(B, Nt, 4), r(B, Nt)
 
 
+@pytest.mark.parametrize("precision,code,cfg", [
+    # head size 16: the contraction and the private pass have no bounded waits, the dense chain is the only one
+    ("bf16", 6, dict(d_model=64, n_heads=4, n_layers=1, d_ff=128)),
+    ("bf16", 6, dict(d_model=64, n_heads=4, n_layers=3, d_ff=256)),
+    ("bf16", 6, dict(d_model=192, n_heads=12, n_layers=2, d_ff=384)),
+    ("fp32", 5, dict(d_model=64, n_heads=4, n_layers=1, d_ff=128)),
+    ("fp32", 5, dict(d_model=128, n_heads=4, n_layers=2, d_ff=256)),
+    ("fp32", 5, dict(d_model=192, n_heads=6, n_layers=2, d_ff=768)),
+])
+def test_dense_chain_gives_up_and_the_next_call_is_correct(precision, code, cfg):
+    """The few-row (6) and the register-tiled chain (5), with a limit of one cycle."""
+    from ar_tabpfn import _lib
+    lib = _lib.lib()
+    p = _network(precision, **cfg)
+    args = _rows(5, 70, 9)
+    good = p.evaluate_joint_density(*args).clone()
+    assert p.last_status() == 0 and bool(good.isfinite().all())
+    try:
+        _lib.check(lib.artab_debug_set(_lib.DEBUG_WAIT_CYCLES, 1))
+        p.evaluate_joint_density(*args)
+        torch.cuda.synchronize()
+    finally:
+        lib.artab_debug_set(_lib.DEBUG_WAIT_CYCLES, 0)
+    assert p.last_status() == code
+    with pytest.raises(_lib.ArtabError, match="wait gave up"):
+        p.evaluate_joint_density(*args)
+    assert torch.equal(p.evaluate_joint_density(*args), good)
+    assert p.last_status() == 0
+
+
 @pytest.mark.parametrize("B,heads,Nc", [(1, 4, 40), (130, 4, 1100), (40, 8, 33), (9, 12, 70)])
 def test_whole_sequence_decode_gives_up_and_the_next_one_is_correct(B, heads, Nc):
     """A limit of one cycle: the first wait for a copy or a peer that has not arrived yet ends the job in every CTA."""
