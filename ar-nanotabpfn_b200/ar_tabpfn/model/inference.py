@@ -405,9 +405,10 @@ class ARTabPFNPredictor:
         K = int(self.head.num_components)
         if expo.shape != (Nt, B, K) or normal.shape != (Nt, B):
             raise ValueError("variates must be (expo [Nt,B,K], normal [Nt,B])")
-        samples = torch.empty(B, Nt, device=device, dtype=torch.float32)
-        logdens = torch.empty(B, Nt, device=device, dtype=torch.float32)
-        comp = torch.empty(B, Nt, device=device, dtype=torch.int32)
+        # zeros: a call whose bounded wait gives up leaves no values of an earlier one in them
+        samples = torch.zeros(B, Nt, device=device, dtype=torch.float32)
+        logdens = torch.zeros(B, Nt, device=device, dtype=torch.float32)
+        comp = torch.zeros(B, Nt, device=device, dtype=torch.int32)
         st = self._state
         stream = _lib.stream_ptr()
 

@@ -227,3 +227,24 @@ def test_whole_sequence_decode_gives_up_and_the_next_one_is_correct(B, heads, Nc
     assert code == 4 and bool((void == -7.0).all())
     again, code = decode()
     assert code == 0 and torch.equal(again, good)
+
+
+@pytest.mark.parametrize("precision,d_ff", [("fp32", 256), ("bf16", 128)])
+def test_results_of_a_sampling_call_that_gave_up_are_zero(precision, d_ff):
+    """Not what an earlier call left in the same memory."""
+    from ar_tabpfn import _lib
+    lib = _lib.lib()
+    p = _network(precision, d_model=64, n_heads=4, n_layers=2, d_ff=d_ff)
+    B, Nt = 6, 11
+    xc, yc, xt, _ = _rows(B, 50, Nt)
+    variates = torch.rand(Nt, B, 5, device="cuda") + 0.1, torch.randn(Nt, B, device="cuda")
+    p.sample_sequence(xc, yc, xt, variates=variates)
+    torch.cuda.synchronize()
+    try:
+        _lib.check(lib.artab_debug_set(_lib.DEBUG_WAIT_CYCLES, 1))
+        void = p.sample_sequence(xc, yc, xt, variates=variates)
+        torch.cuda.synchronize()
+    finally:
+        lib.artab_debug_set(_lib.DEBUG_WAIT_CYCLES, 0)
+    assert p.last_status() != 0
+    assert not bool(void.any()) and not bool(p.last_logdens.any()) and not bool(p.last_components.any())
