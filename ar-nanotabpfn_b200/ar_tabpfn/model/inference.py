@@ -342,6 +342,16 @@ class ARTabPFNPredictor:
             normal[t].normal_()   # the same fill as torch.randn(batch, 1, 1, 1): same element count, same stream
         return expo, normal
 
+    def _sequence_workspace(self, need: int) -> Optional[Tensor]:
+        """Memory of the one-launch decode for the length of a call (up to 4 GiB: nothing a predictor should
+        sit on).  None where it does not apply or does not fit: the decode then goes step by step."""
+        if need <= 0:
+            return None
+        try:
+            return torch.empty(need, dtype=torch.uint8, device=self._device)
+        except torch.cuda.OutOfMemoryError:
+            return None
+
     @torch.no_grad()
     def sample_sequence(self, x_context: Tensor, y_context: Tensor, x_target: Tensor,
                         variates: Optional[Tuple[Tensor, Tensor]] = None) -> Tensor:
@@ -418,20 +428,19 @@ class ARTabPFNPredictor:
                 issue_draws(t + 16)
                 torch.cuda.current_stream(device).wait_event(drawn[t])
 
-        need = int(lib.artab_sequence_workspace(pm.ref, C.byref(st)))
-        if need > 0:
+        ws = self._sequence_workspace(int(lib.artab_sequence_workspace(pm.ref, C.byref(st))))
+        if ws is not None:
             # one launch per chunk of draws (one in all when they are given)
             if x_target.is_cuda and B > 1 and x_target.stride(0) == 0:
                 xt, xt_stride = self._dev32(x_target[:1], device), 0   # the same rows for every stream
             else:
                 xt, xt_stride = self._dev32(x_target, device), Nt * F
-            ws = self._alloc("seq_ws", (need,), torch.uint8)
             for t in range(0, Nt, 16 if drawn is not None else Nt):
                 variates_ready(t)
                 t1 = min(t + 16, Nt) if drawn is not None else Nt
                 _lib.check(lib.artab_decode_sequence(pm.ref, C.byref(st), _lib.ptr(xt), xt_stride, F, Nt, t, t1,
                                                      _lib.ptr(samples), _lib.ptr(expo), _lib.ptr(normal),
-                                                     _lib.ptr(logdens), _lib.ptr(comp), _lib.ptr(ws), need, stream))
+                                                     _lib.ptr(logdens), _lib.ptr(comp), _lib.ptr(ws), ws.numel(), stream))
         else:
             xt = self._dev32(x_target, device)
             for t in range(Nt):

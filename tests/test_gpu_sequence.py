@@ -72,3 +72,36 @@ def test_sequence_matches_oracle(case, precision):
         err = (got.double() - want.double()).abs()
         bound = bar * (1 + want.double().abs()) + 4 * noise
         assert bool((err <= bound).all()), (k, float(err.max()), float((err / bound).max()))
+
+
+def test_workspace_is_given_back_and_a_job_that_has_no_room_for_it_still_runs(monkeypatch):
+    import ar_tabpfn
+    torch.manual_seed(4)
+    m = ar_tabpfn.ARTabPFN(num_features=5).eval().cuda()
+    pred = ar_tabpfn.ARTabPFNPredictor.from_trained_model(m, backend="triton_shared_context", precision="fp32")
+    B, Nc, Nt, K = 9, 2000, 5, 5
+    g = torch.Generator(device="cuda").manual_seed(1)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    expo = torch.rand(Nt, B, K, device="cuda", generator=g) + 0.5
+    expo.scatter_(2, torch.randint(K, (Nt, B, 1), device="cuda", generator=g), 1e-5)
+    args = r(1, Nc, 5).expand(B, -1, -1), r(1, Nc).expand(B, -1), r(1, Nt, 5).expand(B, -1, -1)
+    run = lambda: pred.sample_sequence(*args, variates=(expo, normal))
+    normal = r(Nt, B)
+    asked = []
+    plain = type(pred)._sequence_workspace
+    monkeypatch.setattr(type(pred), "_sequence_workspace", lambda self, need: asked.append(need) or plain(self, need))
+    want = run().clone()
+    assert asked[-1] > 1 << 20
+    held = torch.cuda.memory_allocated()
+    run()
+    assert torch.cuda.memory_allocated() <= held and not any(t.dtype == torch.uint8 for t in pred._bufs.values())
+    monkeypatch.undo()
+
+    def no_room(n, *a, dtype=None, **k):
+        if dtype is torch.uint8:
+            raise torch.cuda.OutOfMemoryError("no room")
+        return empty(n, *a, dtype=dtype, **k)
+    empty = torch.empty
+    monkeypatch.setattr(torch, "empty", no_room)
+    got = run()
+    torch.testing.assert_close(got, want, atol=1e-4, rtol=1e-4)   # fp32 sums in another order, five targets deep
