@@ -25,47 +25,36 @@ def _split_bf16(w: torch.Tensor):
     return hi, lo
 
 
-def _swizzle_block(blk: torch.Tensor) -> torch.Tensor:
-    """[rows][64] bf16 -> the 128-byte-swizzled K-major shared-memory image of that block:
+def _swizzle(blocks: torch.Tensor) -> torch.Tensor:
+    """[..., rows][64] bf16 -> the 128-byte-swizzled K-major shared-memory image of every [rows][64] block:
     16-byte chunk c of row r is stored at chunk position c ^ (r % 8)."""
-    rows = blk.shape[0]
-    chunks = blk.reshape(rows, 8, 8)
-    pos = torch.arange(8, device=blk.device)[None, :] ^ (torch.arange(rows, device=blk.device)[:, None] % 8)
-    out = torch.empty_like(chunks)
-    out.scatter_(1, pos[:, :, None].expand(rows, 8, 8), chunks)
-    return out.reshape(-1)
+    r = torch.arange(8)[:, None]
+    return blocks.reshape(-1, 8, 8, 8)[:, r, torch.arange(8)[None, :] ^ r].reshape(-1)
 
 
-def tile_weight(w: torch.Tensor, mode: str, force_lo: bool = False):
-    """Tile an nn.Linear weight [N][K] (fp64) for the tensor-core chain.
+def tile_weight(hi: torch.Tensor, lo: torch.Tensor, mode: str, force_lo: bool = False):
+    """Tile the hi and lo part of an nn.Linear weight [N][K] for the tensor-core chain.
 
     The result is the exact byte stream the kernel's weight ring consumes: a sequence of
     slabs, each a stack of swizzled [rows][64 k] blocks, hi part then (optionally) lo part.
       mode "full":   one slab per 64-wide k-chunk holding all N rows            (N = d_model)
       mode "ntile":  per 128-row output tile one 16 KB slab per k-chunk         (hidden GEMMs)
     Returns (flat bf16 tensor, has_lo)."""
-    N, K = w.shape
+    N, K = hi.shape
     assert K % 64 == 0
-    hi, lo = _split_bf16(w)
     has_lo = force_lo or bool((lo != 0).any())
-    slabs = []
+    parts = torch.stack((hi, lo) if has_lo else (hi,))
     if mode == "full":
-        for kc in range(K // 64):
-            for part in ((hi, lo) if has_lo else (hi,)):
-                slabs.append(_swizzle_block(part[:, kc * 64:(kc + 1) * 64].contiguous()))
-    else:
-        assert N % 128 == 0
-        for j in range(N // 128):
-            for part in ((hi, lo) if has_lo else (hi,)):
-                for kc in range(K // 64):
-                    slabs.append(_swizzle_block(part[j * 128:(j + 1) * 128, kc * 64:(kc + 1) * 64].contiguous()))
-    return torch.cat(slabs), has_lo
+        return _swizzle(parts.reshape(-1, N, K // 64, 64).permute(2, 0, 1, 3)), has_lo
+    assert N % 128 == 0
+    return _swizzle(parts.reshape(-1, N // 128, 128, K // 64, 64).permute(1, 0, 3, 2, 4)), has_lo
 
 
 class PackedModel:
     """All packing arithmetic (transposes, the fold of the feature attention, hi / lo splits,
-    swizzled tiles) runs on the host in fp64, once per model version; the device sees two copies
-    (the fp32 buffer and the bf16 tile stream) and no packing kernels."""
+    swizzled tiles) runs on the host in fp64, once per model version, and no packing kernels on the device.
+    Each layout is made when the first call needs it (``prepare``, ``prepare_sequence``): new weights cost a
+    call only what it reads."""
 
     def __init__(self, embedder, backbone, head, ar_tokens, device: torch.device):
         target, device = device, torch.device("cpu")
@@ -139,46 +128,79 @@ class PackedModel:
             setattr(m, f, P(f))
         m.layers = C.cast(self._layers, C.POINTER(_lib.LayerWeights))
         self.struct = m
-        self._pack_tensor_core(embedder, backbone, head, target)
-        self._pack_sequence(dict(items), target)
-        self._pack_panels(dict(items), target)
-        self._pack_fragments(dict(items), target)
+        self.tc_flat = self.seq_flat = self.fma_flat = self.mma_flat = None
+        self._w = dict(items)
+        self._target = target
+        self._made = set()
+        self._split = {}
+        D, Dff, H = self.d_model, self.d_ff, self.n_heads
+        ranks = max(c for c in range(1, 9) if H % c == 0)
+        if D % 64 == 0 and Dff % ranks == 0 and D // ranks % 16 == 0 and Dff // ranks % 32 == 0:
+            m.seq_ranks = ranks      # what artab_sequence_workspace goes by; the stream itself: prepare_sequence
 
-    def _pack_tensor_core(self, embedder, backbone, head, target):
+    def _once(self, name: str, make) -> None:
+        if name not in self._made:
+            make(self._w, self._target)
+            self._made.add(name)
+
+    def _halves(self, name: str):
+        """bf16 hi and lo part of a matrix ("wb16": head.2 with 16 output columns), split all together once."""
+        if not self._split:
+            names = [n for n in self._w if n.endswith(("wf_t", "wqkv_t", "wo_t", "w1_t", "w2_t", "wa_t"))] + ["wb16"]
+            wb = torch.zeros(self.d_ff, 16, dtype=torch.float64)
+            wb[:, :3 * self.n_comp] = self._w["wb_t"]
+            mats = [self._w[n] if n != "wb16" else wb for n in names]
+            hi, lo = _split_bf16(torch.cat([m.reshape(-1) for m in mats]))
+            for n, m, h, l in zip(names, mats, hi.split([m.numel() for m in mats]), lo.split([m.numel() for m in mats])):
+                self._split[n] = h.view(m.shape), l.view(m.shape)
+        return self._split[name]
+
+    def prepare(self, bf16: bool) -> "PackedModel":
+        """Lay the weights out for the dense chains of this precision."""
+        if bf16:
+            self._once("tensor_core", self._pack_tensor_core)
+        if bf16 and self.tc_flat is not None:
+            self._once("fragments", self._pack_fragments)
+            self._split = {}
+        else:
+            self._once("panels", self._pack_panels)
+        return self
+
+    def prepare_sequence(self) -> None:
+        """Lay the weights out for artab_decode_sequence."""
+        if self.struct.seq_ranks:
+            self._once("sequence", self._pack_sequence)
+
+    def _pack_tensor_core(self, w, target):
         """bf16 hi/lo tiles for the tcgen05 per-token chain (d_model in {64,128,192}, d_ff % 128 == 0,
         3K <= 16).  Other shapes keep the fp32 FMA chain (the tc_* pointers stay NULL)."""
         D, Dff = self.d_model, self.d_ff
         device = torch.device("cpu")
-        self.tc_flat = None
         if D not in (64, 128, 192) or Dff % 128 != 0 or Dff > 1024 or 3 * self.n_comp > 16:
             return
-        f64 = lambda t: t.detach().to(device=device, dtype=torch.float64)
         items = []
 
-        def add(name, w, mode, force_lo=False):
-            flat, has_lo = tile_weight(w, mode, force_lo)
+        def add(name, parts, mode, force_lo=False):   # parts: hi, lo [in][out]
+            flat, has_lo = tile_weight(parts[0].t(), parts[1].t(), mode, force_lo)
             items.append((name, flat))
             return has_lo
 
         layer_lo = []
-        for i, l in enumerate(backbone.layers):
-            r = l.attn_rows
+        for i in range(self.n_layers):
             bits = 0
-            bits |= 1 * add(f"{i}.tc_wo", f64(r.out_proj.weight), "full")
-            bits |= 2 * add(f"{i}.tc_w1", f64(l.ff[0].weight), "ntile")
-            bits |= 4 * add(f"{i}.tc_w2", f64(l.ff[2].weight), "full")
-            wf = f64(l.attn_features.out_proj.weight) @ f64(l.attn_features.v_proj.weight)
-            bits |= 8 * add(f"{i}.tc_wf", wf, "full")
+            bits |= 1 * add(f"{i}.tc_wo", self._halves(f"{i}.wo_t"), "full")
+            bits |= 2 * add(f"{i}.tc_w1", self._halves(f"{i}.w1_t"), "ntile")
+            bits |= 4 * add(f"{i}.tc_w2", self._halves(f"{i}.w2_t"), "full")
+            bits |= 8 * add(f"{i}.tc_wf", self._halves(f"{i}.wf_t"), "full")
             # q, k, v must agree on the lo part: they share one flag
-            qkv_lo = any(bool((_split_bf16(f64(p.weight))[1] != 0).any()) for p in (r.q_proj, r.k_proj, r.v_proj))
-            for nm, p in (("q", r.q_proj), ("k", r.k_proj), ("v", r.v_proj)):
-                add(f"{i}.tc_w{nm}", f64(p.weight), "full", force_lo=qkv_lo)
+            hi, lo = self._halves(f"{i}.wqkv_t")
+            qkv_lo = bool((lo != 0).any())
+            for j, nm in enumerate("qkv"):
+                add(f"{i}.tc_w{nm}", (hi[:, j * D:(j + 1) * D], lo[:, j * D:(j + 1) * D]), "full", force_lo=qkv_lo)
             bits |= 16 * qkv_lo
             layer_lo.append(bits)
-        head_bits = 1 * add("tc_wa", f64(head.head[0].weight), "ntile")
-        wb = torch.zeros(16, Dff, dtype=torch.float64, device=device)
-        wb[: 3 * self.n_comp] = f64(head.head[2].weight)
-        head_bits |= 2 * add("tc_wb", wb, "full")
+        head_bits = 1 * add("tc_wa", self._halves("wa_t"), "ntile")
+        head_bits |= 2 * add("tc_wb", self._halves("wb16"), "full")
         offs, tot = {}, 0
         for name, t in items:
             offs[name] = tot
@@ -206,43 +228,31 @@ class PackedModel:
         order of use (layer by layer: fold, Q|K|V of the rank's heads | out-projection, MLP; then the head).
         A slice [K][N] is a sequence of units of 32 k x 16 columns, k blocks outermost; inside a unit element
         (k = 4s + e, n = 4g + c) sits at [c][s][g][e].  ``w`` holds the matrices as [in][out]."""
-        D, Dff, H, Dh, K = self.d_model, self.d_ff, self.n_heads, self.head_dim, self.n_comp
-        ranks = max(c for c in range(1, 9) if H % c == 0)
-        self.seq_flat = None
-        if D % 64 or Dff % ranks or D // ranks % 16 or Dff // ranks % 32:
-            return
-        ds, hs, qs = D // ranks, Dff // ranks, H // ranks * Dh
+        D, Dff, K = self.d_model, self.d_ff, self.n_comp
+        ranks = self.struct.seq_ranks
+        hs, L = Dff // ranks, self.n_layers
         wb = torch.zeros(Dff, (3 * K + 15) // 16 * 16, dtype=torch.float64)
         wb[:, :3 * K] = w["wb_t"]
-        unit = lambda m: (m.reshape(m.shape[0] // 32, 8, 4, m.shape[1] // 16, 4, 4).permute(0, 3, 5, 1, 4, 2)
-                          .to(torch.float32).reshape(-1))
-        streams = []
-        for r in range(ranks):
-            cols = lambda m, n: m[:, r * n:(r + 1) * n]
-            parts = []
-
-            def pre(i):
-                parts.append(cols(w[f"{i}.wf_t"], ds))
-                parts.append(torch.cat([cols(m, qs) for m in w[f"{i}.wqkv_t"].split(D, dim=1)], dim=1))
-
-            pre(0)
-            for i in range(self.n_layers):
-                parts += [cols(w[f"{i}.wo_t"], ds), cols(w[f"{i}.w1_t"], hs), w[f"{i}.w2_t"][r * hs:(r + 1) * hs]]
-                if i + 1 < self.n_layers:
-                    pre(i + 1)
-            parts += [cols(w["wa_t"], hs), wb[r * hs:(r + 1) * hs]]
-            # after the matrices: per layer LayerNorm 1 / 2 vectors, b2, LayerNorm 3 vectors, b1 slice; final
-            # LayerNorm, first bias of the head (slice)
-            part = lambda v: v[r * hs:(r + 1) * hs]
-            vec = []
-            for i in range(self.n_layers):
-                vec += [w[f"{i}.{k}"] for k in ("ln1_g", "ln1_b", "ln2_g", "ln2_b", "b2", "ln3_g", "ln3_b")] + [part(w[f"{i}.b1"])]
-            vec += [w["lnf_g"], w["lnf_b"], part(w["ba"])]
-            mats = [unit(p) for p in parts]
-            self.struct.seq_vec_off = 4 * sum(m.numel() for m in mats)
-            streams.append(torch.cat(mats + [v.reshape(-1).to(torch.float32) for v in vec]))
-        flat = torch.stack(streams)
-        self.struct.seq_ranks = ranks
+        f32 = lambda m: m.to(torch.float32)
+        # -> [rank][units of its slice]
+        cols = lambda m: (f32(m).reshape(m.shape[0] // 32, 8, 4, ranks, m.shape[1] // ranks // 16, 4, 4)
+                          .permute(3, 0, 4, 6, 1, 5, 2).reshape(ranks, -1))
+        rows = lambda m: f32(m).reshape(ranks, hs // 32, 8, 4, m.shape[1] // 16, 4, 4).permute(0, 1, 4, 6, 2, 5, 3).reshape(ranks, -1)
+        by_rank = lambda m: m.reshape(D, 3, ranks, D // ranks).transpose(1, 2).reshape(D, 3 * D)   # q | k | v of a rank together
+        mats = []
+        for i in range(L):
+            mats += [cols(w[f"{i}.wf_t"]), cols(by_rank(w[f"{i}.wqkv_t"]))]
+            mats += [cols(w[f"{i}.wo_t"]), cols(w[f"{i}.w1_t"]), rows(w[f"{i}.w2_t"])]
+        mats += [cols(w["wa_t"]), rows(wb)]
+        self.struct.seq_vec_off = 4 * sum(m.shape[1] for m in mats)
+        # after the matrices: per layer LayerNorm 1 / 2 vectors, b2, LayerNorm 3 vectors, b1 slice; final
+        # LayerNorm, first bias of the head (slice)
+        whole = lambda v: f32(v).reshape(1, -1).expand(ranks, -1)
+        part = lambda v: f32(v).reshape(ranks, hs)
+        for i in range(L):
+            mats += [whole(w[f"{i}.{k}"]) for k in ("ln1_g", "ln1_b", "ln2_g", "ln2_b", "b2", "ln3_g", "ln3_b")] + [part(w[f"{i}.b1"])]
+        mats += [whole(w["lnf_g"]), whole(w["lnf_b"]), part(w["ba"])]
+        flat = torch.cat(mats, dim=1)
         self.struct.seq_rank_bytes = 4 * flat.shape[1]
         self.seq_flat = flat.to(target)
         self.struct.seq_w = self.seq_flat.data_ptr()
@@ -250,7 +260,6 @@ class PackedModel:
     def _pack_panels(self, w, target):
         """D x D panels of every matrix for the register-tiled fp32 chain, in the order it uses them."""
         D, Dff, K = self.d_model, self.d_ff, self.n_comp
-        self.fma_flat = None
         if D not in (64, 128, 192) or Dff % D or Dff > 1024 or 3 * K > D:
             return
         chunks = range(0, Dff, D)
@@ -275,29 +284,27 @@ class PackedModel:
         """mma.m16n8k16 B fragments for the few-row bf16 chain: four slices of every matrix (by output column, w2 and
         head.2 by input row), hi part then lo part.  A part is a sequence of units of 8 columns x 32 k, k innermost;
         in a unit lane (g, t) holds column g, k = 16 ks + 8 half + 2 t + e at [ks][half][e]."""
-        self.mma_flat = None
-        if self.tc_flat is None:
-            return
         D, Dff, K = self.d_model, self.d_ff, self.n_comp
-        ds, hs = D // 4, Dff // 4
-        wb = torch.zeros(Dff, 16, dtype=torch.float64)
-        wb[:, :3 * K] = w["wb_t"]
+        hs = Dff // 4
 
-        def parts(m):
-            u = lambda t: t.reshape(m.shape[0] // 32, 2, 2, 4, 2, m.shape[1] // 8, 8).permute(5, 0, 6, 3, 1, 2, 4).reshape(-1)
-            hi, lo = _split_bf16(m)
-            return [u(hi.to(torch.bfloat16)), u(lo.to(torch.bfloat16))]
+        # -> the hi and the lo part, each [rank][fragment order]
+        def cols(name):
+            ms = self._halves(name)
+            if name.endswith("wqkv_t"):   # q | k | v of a rank together
+                ms = [m.reshape(D, 3, 4, D // 4).transpose(1, 2).reshape(D, 3 * D) for m in ms]
+            k, n = ms[0].shape
+            return [m.reshape(k // 32, 2, 2, 4, 2, 4, n // 32, 8).permute(5, 6, 0, 7, 3, 1, 2, 4).reshape(4, -1) for m in ms]
 
-        def streams(matrices):
-            return torch.cat([p for r in range(4) for m in matrices(r) for p in parts(m.contiguous())])
+        def rows(name):
+            ms = self._halves(name)
+            return [m.reshape(4, hs // 32, 2, 2, 4, 2, m.shape[1] // 8, 8).permute(0, 6, 1, 7, 4, 2, 3, 5).reshape(4, -1) for m in ms]
 
-        cols = lambda m, r: m[:, r * m.shape[1] // 4:(r + 1) * m.shape[1] // 4]
-        rows = lambda m, r: m[r * hs:(r + 1) * hs]
+        streams = lambda *parts: torch.cat(sum(parts, []), dim=1).reshape(-1)
         stacks = []
         for i in range(self.n_layers):
-            stacks.append(streams(lambda r: [cols(w[f"{i}.wf_t"], r), torch.cat([cols(m, r) for m in w[f"{i}.wqkv_t"].split(D, dim=1)], dim=1)]))
-            stacks.append(streams(lambda r: [cols(w[f"{i}.wo_t"], r), cols(w[f"{i}.w1_t"], r), rows(w[f"{i}.w2_t"], r)]))
-        stacks.append(streams(lambda r: [cols(w["wa_t"], r), rows(wb, r)]))
+            stacks.append(streams(cols(f"{i}.wf_t"), cols(f"{i}.wqkv_t")))
+            stacks.append(streams(cols(f"{i}.wo_t"), cols(f"{i}.w1_t"), rows(f"{i}.w2_t")))
+        stacks.append(streams(cols("wa_t"), rows("wb16")))
         self.mma_flat = torch.cat(stacks).to(target)
         at = self.mma_flat.data_ptr()
         for n, st in enumerate(stacks):

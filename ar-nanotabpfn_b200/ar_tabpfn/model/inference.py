@@ -83,7 +83,8 @@ class ARTabPFNPredictor:
         return self.backend == "triton_shared_context"
 
     def _packed(self, device):
-        return packed_for(self, self.embedder, self.backbone, self.head, self.ar_tokens, device)
+        pm = packed_for(self, self.embedder, self.backbone, self.head, self.ar_tokens, device)
+        return pm.prepare(self._cache_dtype(self._dtype) == torch.bfloat16)
 
     def _cache_dtype(self, dtype: Optional[torch.dtype]) -> torch.dtype:
         if self.precision == "fp32":
@@ -430,6 +431,7 @@ class ARTabPFNPredictor:
 
         ws = self._sequence_workspace(int(lib.artab_sequence_workspace(pm.ref, C.byref(st))))
         if ws is not None:
+            pm.prepare_sequence()
             # one launch per chunk of draws (one in all when they are given)
             if x_target.is_cuda and B > 1 and x_target.stride(0) == 0:
                 xt, xt_stride = self._dev32(x_target[:1], device), 0   # the same rows for every stream

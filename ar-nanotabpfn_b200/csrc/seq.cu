@@ -92,7 +92,7 @@ size_t context_bytes(const artab_model* m, const artab_state* st) {
 
 bool seq_plan(const artab_model* m, const artab_state* st, SeqPlan& p, SeqArgs& a) {
   const int D = m->d_model, DH = m->head_dim, H = m->n_heads;
-  if (!m->seq_w || m->seq_ranks <= 0 || m->n_layers > kSeqMaxLayers || m->n_comp > 32) return false;
+  if (m->seq_ranks <= 0 || m->n_layers > kSeqMaxLayers || m->n_comp > 32) return false;
   const int C = largest_divisor(H, 8);
   // a CTA of its own has no cluster to st.async into: the one launch of this kernel without a cluster
   // dimension (one head) ended in an illegal instruction
@@ -176,6 +176,7 @@ int launch_seq(const artab_model* m, const artab_state* st, const SeqCall& c, cu
   SeqArgs a;
   memset(&a, 0, sizeof(a));
   ARTAB_REQUIRE(seq_plan(m, st, p, a), ARTAB_EINVAL, "decode_sequence: not available for this model");
+  ARTAB_REQUIRE(m->seq_w, ARTAB_EINVAL, "decode_sequence: the weight streams (seq_w) are missing");
   ARTAB_REQUIRE(c.workspace_bytes >= context_bytes(m, st), ARTAB_ECAPACITY, "decode_sequence: workspace too small");
   const bool bf = st->dtype == ARTAB_BF16;
   if (c.t0 == 0) {  // first part of a sequence: the context is new

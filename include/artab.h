@@ -124,9 +124,10 @@ typedef struct artab_model {
   int32_t tc_reserved;
   const artab_layer_weights* layers; /* HOST pointer to n_layers entries */
   const float* fma_head;             /* per D-wide chunk j: wa[:, j], then wb[j, :] padded to D columns (or NULL) */
-  /* whole-sequence decode (NULL: artab_decode_sequence is not available): per cluster rank one contiguous
-   * stream of the matrix slices that rank uses, in the order of use, fp32 in units of 32 k x 16 columns (_pack.py);
-   * seq_ranks is the largest divisor of n_heads that is at most 8 */
+  /* whole-sequence decode (seq_ranks 0: not available): per cluster rank one contiguous stream of the matrix
+   * slices that rank uses, in the order of use, fp32 in units of 32 k x 16 columns (_pack.py); seq_ranks is the
+   * largest divisor of n_heads that is at most 8; artab_sequence_workspace needs only that, so seq_w may be made
+   * when it is first used */
   const void* seq_w;
   int64_t seq_rank_bytes, seq_vec_off;  /* bytes per rank; where its LayerNorm and bias vectors start */
   int32_t seq_ranks;

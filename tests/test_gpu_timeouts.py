@@ -205,6 +205,7 @@ def test_whole_sequence_decode_gives_up_and_the_next_one_is_correct(B, heads, Nc
     pm, st = p._packed(p._device), p._state
     need = int(lib.artab_sequence_workspace(pm.ref, C.byref(st)))
     assert need > 0
+    pm.prepare_sequence()
     ws, status = torch.empty(need, dtype=torch.uint8, device="cuda"), p._bufs["status"]
 
     def decode():
