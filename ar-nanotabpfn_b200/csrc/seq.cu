@@ -90,6 +90,44 @@ size_t context_bytes(const artab_model* m, const artab_state* st) {
   return (size_t)m->n_layers * st->n_groups * m->n_heads * ((st->n_ctx + 31) / 32) * (64 * (size_t)m->head_dim * 4);
 }
 
+// Which path is faster, from a cost of each: microseconds per layer and target.
+//
+// One launch: a serial chain of phases per layer that grows with d_model and with the rows of the kernel variant, the
+// walk of the head's context keys by one CTA, the context laid out again once per job, the head and the sampler per
+// target.  A launch per layer: a chain that hardly notices the rows, and a contraction whose keys are split over the
+// chip, bounded by the walk of a split (at most 16), by FMAs or by the bytes of the streams' own contexts.
+//
+// The constants are fitted to 856 points where both ran: d_model 64 - 192, 2 - 12 heads, 2 - 12 layers, fp32 and bf16,
+// 1 - 400 streams on one context of 128 - 16384 rows or 4 - 250 own ones of 100 - 6000, 8 - 64 targets.  Of these the
+// path picked is never more than 12 % slower than the other one and 0.1 % on average.  One launch against one per
+// layer, us: d_model 128, fp32, 8 streams, 128 rows 12.6 : 45, 1000 rows 15.8 : 48, 4000 rows 29 : 52, 16384 rows
+// 88 : 73; 200 streams, 1000 rows 51 : 58, 4000 rows 121 : 86; d_model 192, bf16, 32 streams, 1000 rows 22 : 30, 4000
+// rows 38 : 33; 64 datasets of 500 rows 37 : 48, of 2000 rows 64 : 77.
+bool faster_in_one_launch(const artab_model* m, const artab_state* st, int C, int spc) {
+  const double D = m->d_model, L = m->n_layers, H = m->n_heads, head = m->head_dim / 32.0;
+  const double B = st->n_streams, keys = st->n_ctx, targets = st->max_buf > 1 ? st->max_buf : 1;
+  const bool shared = st->n_groups == 1, bf = st->dtype == ARTAB_BF16;
+
+  const int variant = spc <= 1 ? 0 : spc <= 2 ? 1 : spc <= 4 ? 2 : 3;   // 2, 4, 8, 16 rows
+  static const double kChain[4] = {1, 1.2, 2.0, 2.6}, kKeys[4] = {4.4e-3, 5.2e-3, 8.3e-3, 28e-3};
+  double one = (5.7 + 0.036 * D) * (variant == 3 && !shared ? 3.5 : kChain[variant]) + 5 / L;
+  one += H / C * head * keys * (shared ? kKeys[variant] : 4.8e-3 * spc);
+  one += (shared ? 1 : B) * D * keys * 8 / 1.3e6 / targets;
+
+  double each = (chain_on_tc(m, st) ? 7 + 0.099 * D : 8 + 0.35 * D) + 21 / L;
+  const double bytes = B * D * keys * (bf ? 6 : 8);                     // own contexts
+  if (ctx_attn_tc_supported(st->dtype, m->head_dim)) {
+    each += shared ? 0.86e-3 * keys : 0.012 * B * H + bytes / 3.6e6;
+  } else {
+    const int rows = 2 * st->n_streams, tiles = (st->n_ctx + 63) / 64;
+    const double walk = keys / (tiles < 16 ? tiles : 16) * head * (rows <= 16 ? 0.022 : rows <= 32 ? 0.027 : 0.054);
+    const double work = shared ? rows * keys * D * 4 / 22e6 : bytes / 1.1e6;
+    each += shared && walk > work ? walk : work;
+    if (bf) each += (shared ? walk : 0.012 * B * H) + 8.9 * (keys < 1000 ? keys / 1000 : 1);
+  }
+  return one < each;
+}
+
 bool seq_plan(const artab_model* m, const artab_state* st, SeqPlan& p, SeqArgs& a) {
   const int D = m->d_model, DH = m->head_dim, H = m->n_heads;
   if (m->seq_ranks <= 0 || m->n_layers > kSeqMaxLayers || m->n_comp > 32) return false;
@@ -115,16 +153,7 @@ bool seq_plan(const artab_model* m, const artab_state* st, SeqPlan& p, SeqArgs& 
   // the re-tiled copy of the context is as large as its fp32 cache: not where that is a good part of the memory
   if (context_bytes(m, st) > kWorkspaceMax) return false;
   const int spc = (st->n_streams + fit - 1) / fit;
-  // Models whose launch-per-layer path runs on tensor cores.  That path hardly notices the number of streams, this
-  // kernel walks up to four rows per cluster at the same speed and more at a lower one (6 layers, d_model 192, 1000
-  // context rows, 8 targets: 1.9 against 2.3 ms at 32 streams, 2.7 against 2.3 at 48); nor does that path notice
-  // the context as much where the contraction is on tensor cores too (24 streams: 2.3 against 2.5 ms at 2000 rows,
-  // 3.0 against 2.7 at 4000).  A context per stream leaves its 128-query tiles nearly empty: 3.5 against 3.9 ms for
-  // 64 datasets of 500 rows, equal at 96.
-  if (chain_on_tc(m, st)) {
-    if (st->n_groups > 1 ? st->n_streams > 64 : spc > 2) return false;
-    if (st->n_groups == 1 && ctx_attn_tc_supported(st->dtype, DH) && st->n_ctx > 3000) return false;
-  }
+  if (!faster_in_one_launch(m, st, C, spc)) return false;
   const int R = spc <= 1 ? 2 : spc <= 2 ? 4 : spc <= 4 ? 8 : kMaxRowsPerCluster;
   const Areas ar = areas_of(m, C, R);
   const size_t fixed = kSeqBarBytes + 4 * ((size_t)ar.red + ar.area);

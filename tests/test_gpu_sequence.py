@@ -1,6 +1,9 @@
 """The one-launch decode of a whole sampling job against the CPU oracle: every kernel variant (streams per
 cluster, head size, cache type, shared or own contexts) at the sizes where its tiles end: context tiles of
-32 keys, private keys of 32 in four parts, clusters with a stream missing, several heads per CTA."""
+32 keys, private keys of 32 in four parts, clusters with a stream missing, several heads per CTA.  Every case says
+whether the one-launch path is to take it."""
+import ctypes
+
 import pytest
 import torch
 
@@ -8,21 +11,35 @@ import artab_oracle as orc
 
 pytestmark = pytest.mark.gpu
 
-# d_model, heads, layers, d_ff, components, streams, context rows, targets, shared
+# d_model, heads, layers, d_ff, components, streams, context rows, targets, shared; one launch in fp32, in bf16
 CASES = [
-    (64, 4, 2, 128, 5, 1, 1, 3, True),          # one key, one stream
-    (64, 4, 1, 128, 20, 5, 33, 6, True),        # head size 16, twenty components
-    (64, 2, 1, 128, 5, 37, 31, 4, True),        # two CTAs per cluster, context one key short of a tile
-    (64, 1, 1, 64, 5, 3, 64, 5, True),          # one head: no cluster to form, the launch-per-layer path
-    (128, 4, 2, 256, 5, 130, 40, 4, True),      # four streams per cluster, the last cluster not full
-    (128, 2, 1, 256, 3, 9, 70, 5, False),       # head size 64, own contexts
-    (128, 8, 1, 512, 5, 200, 30, 3, True),      # eight CTAs, more streams than one wave: the launch-per-layer path
-    (192, 6, 1, 768, 5, 20, 65, 4, False),      # own contexts, head size 32
-    (192, 12, 1, 192, 5, 3, 20, 3, True),       # two heads of 16 per CTA
-    (64, 4, 1, 128, 5, 6, 50, 140, True),       # private keys beyond one round of the four parts
-    (128, 8, 1, 512, 5, 100, 30, 3, True),      # eight CTAs, the widest variant within one wave
-    (64, 4, 1, 128, 8, 250, 20, 3, False),      # the widest variant, a context per stream, clusters not full
-    (64, 4, 1, 128, 5, 420, 20, 3, False),      # the same with a context per stream
+    (64, 4, 2, 128, 5, 1, 1, 3, True, True, True),          # one key, one stream
+    (64, 4, 1, 128, 20, 5, 33, 6, True, True, True),        # head size 16, twenty components
+    (64, 2, 1, 128, 5, 37, 31, 4, True, True, True),        # two CTAs per cluster, context one key short of a tile
+    (64, 1, 1, 64, 5, 3, 64, 5, True, False, False),        # one head: no cluster to form
+    (128, 4, 2, 256, 5, 130, 40, 4, True, True, True),      # four streams per cluster, the last cluster not full
+    (128, 2, 1, 256, 3, 9, 70, 5, False, True, True),       # head size 64, own contexts
+    (128, 8, 1, 512, 5, 200, 30, 3, True, False, False),    # eight CTAs, more streams than one wave
+    (192, 6, 1, 768, 5, 20, 65, 4, False, True, True),      # own contexts, head size 32
+    (192, 12, 1, 192, 5, 3, 20, 3, True, True, True),       # two heads of 16 per CTA
+    (64, 4, 1, 128, 5, 6, 50, 140, True, True, True),       # private keys beyond one round of the four parts
+    (128, 8, 1, 512, 5, 100, 30, 3, True, True, True),      # eight CTAs, the widest variant within one wave
+    (64, 4, 1, 128, 8, 250, 20, 3, False, True, True),      # the widest variant, a context per stream, clusters not full
+    (64, 4, 1, 128, 5, 420, 20, 3, False, False, False),    # four CTAs, a context per stream, more streams than one wave
+    # one context: the 4-, 8- and 16-row variants of each head size (64: no room for 16 rows), most for models
+    # outside the tensor-core chain
+    (64, 4, 1, 128, 20, 60, 33, 3, True, True, True),
+    (64, 4, 1, 128, 20, 130, 40, 3, True, True, True),
+    (64, 4, 2, 128, 20, 199, 65, 3, True, True, True),
+    (128, 4, 1, 256, 20, 70, 33, 3, True, True, True),
+    (128, 4, 1, 256, 8, 107, 31, 3, True, True, True),
+    (128, 4, 1, 256, 5, 201, 64, 3, True, True, True),
+    (128, 4, 1, 256, 20, 201, 64, 3, True, False, False),   # no room for the widest variant
+    (128, 2, 1, 256, 8, 100, 33, 3, True, True, True),
+    (128, 2, 1, 256, 20, 260, 40, 3, True, True, True),
+    # where a launch per layer is the faster one
+    (128, 4, 1, 256, 5, 200, 4000, 2, True, False, False),
+    (64, 2, 2, 128, 5, 3, 6000, 2, True, True, False),
 ]
 
 
@@ -30,7 +47,7 @@ CASES = [
 @pytest.mark.parametrize("case", CASES, ids=lambda c: "d%d_h%d_l%d_ff%d_k%d_b%d_nc%d_nt%d_%s" % (*c[:8], "shared" if c[8] else "own"))
 def test_sequence_matches_oracle(case, precision):
     import ar_tabpfn
-    D, H, L, Dff, K, B, Nc, Nt, shared = case
+    D, H, L, Dff, K, B, Nc, Nt, shared = case[:9]
     torch.manual_seed(3 + D + Nc)
     m = ar_tabpfn.ARTabPFN(d_model=D, n_heads=H, n_layers=L, d_ff=Dff, num_features=5, num_components=K).eval()
     r = lambda t: t.to(torch.bfloat16).float()
@@ -56,6 +73,9 @@ def test_sequence_matches_oracle(case, precision):
     got_y = pred.sample_sequence(c(xc), c(yc), c(xt), variates=(c(expo), c(normal))).cpu()
     got_ld = pred.last_logdens.cpu()
     assert pred.last_status() == 0
+    from ar_tabpfn import _lib
+    one_launch = _lib.lib().artab_sequence_workspace(pred._packed(pred._device).ref, ctypes.byref(pred._state)) > 0
+    assert one_launch == case[10 if precision == "bf16" else 9]
     assert torch.equal(pred.last_components.cpu(), want_c)
     # Bounds: the bar of the mode plus four times what the mode's arithmetic moves the oracle itself by on
     # this stream (root mean square over its targets): fp32 against fp64; bf16 storage of q / k / v and bf16
