@@ -205,7 +205,7 @@ int run_ctx(const artab_model* m, const artab_state* st, int layer, int rows, in
   c.lse = lse;
   c.status = st->status;
   c.kv_stable = kv_stable ? 1 : 0;
-  return use_tc(st->dtype, m->head_dim) ? launch_ctx_attn_tc(c, s) : launch_ctx_attn_simt(c, s);
+  return use_tc(st->dtype, m->head_dim) ? launch_ctx_attn_tc(c, s) : launch_ctx_attn_fma(c, s);
 }
 
 void fill_head(const artab_model* m, DenseArgs& d) {
@@ -787,7 +787,7 @@ int artab_context_attention(int dtype, const void* q, const void* k_ctx, const v
   c.lse = lse;
   c.status = status;
   return use_tc(dtype, head_dim) ? launch_ctx_attn_tc(c, (cudaStream_t)stream)
-                                 : launch_ctx_attn_simt(c, (cudaStream_t)stream);
+                                 : launch_ctx_attn_fma(c, (cudaStream_t)stream);
 }
 
 int artab_buffer_attention_merge(int dtype, const void* q, const void* kv_buf, int n_streams, int n_heads,
@@ -940,7 +940,7 @@ int artab_hybrid_attention(int dtype, const void* q, const void* k_ctx, const vo
   int rc;
   {
     PlainLaunchScope plain;  // the caller's earlier launches are unknown: see common.cuh
-    rc = tc ? launch_ctx_attn_tc(c, s) : launch_ctx_attn_simt(c, s);
+    rc = tc ? launch_ctx_attn_tc(c, s) : launch_ctx_attn_fma(c, s);
   }
   if (rc) return rc;
   // The merge may start beside the contraction: what it reads before its wait (queries, private K / V, mask)

@@ -57,7 +57,7 @@ struct BufMergeArgs {
   const int32_t* poison_if;
 };
 
-int launch_ctx_attn_simt(const CtxAttnArgs& a, cudaStream_t s);  // fp32 FMA, head_dim 16 / 32 / 64
+int launch_ctx_attn_fma(const CtxAttnArgs& a, cudaStream_t s);  // fp32 FMA, head_dim 16 / 32 / 64
 int ctx_attn_fma_rows(int rows_in_group);                        // query rows of one of its CTAs
 int launch_ctx_attn_tc(const CtxAttnArgs& a, cudaStream_t s);  // tcgen05, bf16, head_dim 32
 bool ctx_attn_tc_supported(int dtype, int head_dim);

@@ -198,7 +198,7 @@ int ctx_attn_fma_rows(int rows_in_group) {
   return kWarps * (r <= 2 ? 2 : r <= 4 ? 4 : 8);
 }
 
-int launch_ctx_attn_simt(const CtxAttnArgs& a, cudaStream_t s) {
+int launch_ctx_attn_fma(const CtxAttnArgs& a, cudaStream_t s) {
   if (a.rows <= 0) return ARTAB_OK;
   ARTAB_REQUIRE(a.n_ctx > 0 && a.n_splits >= 1, ARTAB_EINVAL, "context attention: empty context or no splits");
   ARTAB_REQUIRE(a.head_dim == 16 || a.head_dim == 32 || a.head_dim == 64, ARTAB_EINVAL,

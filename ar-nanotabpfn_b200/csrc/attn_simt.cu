@@ -24,7 +24,7 @@ __device__ __forceinline__ float fast_exp2(float x) {  // MUFU ex2: relative err
 // ---------------------------------------------------------------------------
 template <typename T, int DH, bool OP>   // OP: the operator form, see buf_mma_kernel; one query row per item
 __global__ void __launch_bounds__(128, 6) buf_merge_kernel(const BufMergeArgs a) {
-  dep_trigger();  // the dependent dense chain reads only model constants before its wait (see buf_mma_kernel)
+  dep_trigger();  // the dependent reads at most model constants before its wait (see common.cuh)
   constexpr int VEC = Vec16<T>::N;
   constexpr int LPK = DH / VEC;   // lanes per key
   constexpr int KPI = 32 / LPK;   // keys per warp iteration

@@ -70,8 +70,8 @@ template <bool OP>
 __global__ void __launch_bounds__(WPB * 32, 6) buf_mma_kernel(const BufMergeArgs a) {
   __shared__ __align__(16) uint8_t vs[WPB][NR][KB * PITCH];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // The dependent of this kernel is always a dense chain, which reads nothing but model constants
-  // before its own wait: it may become resident (barriers, tensor-memory allocation, first weight
+  // The dependent of this kernel is a dense chain, which reads nothing but model constants
+  // before its own wait (behind the operator form: see common.cuh): it may become resident (barriers, tensor-memory allocation, first weight
   // tiles) while this kernel is still walking the private buffers.  Its wait still covers everything
   // older, because this grid only completes after its own wait below.
   dep_trigger();

@@ -28,21 +28,27 @@ void prof_end(cudaStream_t s);
 // Rules every such kernel follows: (1) it calls dep_wait() before it reads anything an earlier
 // kernel wrote and before it writes global memory; (2) it calls dep_trigger() only after its own
 // dep_wait(), so a dependent that starts early knows that everything older than its predecessor
-// has completed.  One exception to (2): the buffer-pass kernels trigger at their start, because
-// their dependent is always a dense chain, which touches only model constants before its own wait
-// (and that wait still covers everything older: a buffer-pass grid completes only after its own
-// wait).  Without the launch attribute both calls are no-ops.
+// has completed.  One exception to (2): the buffer-pass kernels trigger at their start.  Their
+// dependent is a dense chain, which touches only model constants before its own wait, or, behind the
+// operator form, the first kernel of whatever call comes next: a plain launch or an embedder, which waits
+// first.  (That wait covers everything older: a buffer-pass grid completes only after its own wait.)
+// Without the launch attribute both calls are no-ops.
 //
 // What each kernel reads BEFORE its dep_wait() (the work it overlaps with its predecessor):
 //   embed_kernel            nothing
 //   dense_tc_kernel         weight tiles, LayerNorm vectors and biases (model constants)
+//   dense_mma_kernel        the first weight fragments, LayerNorm vectors and biases (model constants)
+//   retile_kernel,
+//   seq_simt_kernel         nothing
 //   ctx_attn_tc_kernel      context K / V tiles, only when the caller says they are stable (kv_stable)
 //   buf_mma_kernel /
 //   buf_merge_kernel        q, the private K / V rows and the per-stream lengths
+// (the other kernels, dense_fma_kernel and ctx_attn_fma_kernel among them, are launched plainly).
 // The last line is safe only where the launch BEFORE the predecessor produced q and the K / V rows,
 // which holds inside artab_prefill / artab_decode_step / artab_teacher_forcing / artab_forward_masked
 // (embed, dense chain, context contraction, buffer pass: the buffer pass's predecessor is the context
-// contraction, which waits before it triggers).  The single-operator entry points cannot know what
+// contraction, which waits before it triggers), and in artab_hybrid_attention, whose contraction is a plain
+// launch: it starts after everything the merge reads early is complete.  The other single-operator entry points cannot know what
 // the caller launched before them, so they launch every kernel plainly (PlainLaunchScope): the
 // kernel then starts after everything earlier in the stream has completed and the rule is moot.
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -71,6 +71,6 @@ int launch_dense_mma(const DenseArgs& a, cudaStream_t s); // bf16 chain for few 
 bool dense_mma_applicable(const DenseArgs& a);
 bool dense_fma_applicable(const DenseArgs& a);
 bool dense_tc_applicable(const DenseArgs& a);
-bool chain_on_tc(const artab_model* m, const artab_state* st);  // every dense launch of this model takes the tcgen05 chain
+bool chain_on_tc(const artab_model* m, const artab_state* st);  // every dense launch of this model takes the tcgen05 or the few-row chain
 
 }  // namespace artab

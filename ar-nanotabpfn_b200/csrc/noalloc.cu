@@ -89,7 +89,7 @@ extern "C" ARTAB_API int artab_context_attention_noalloc(int dtype, const void* 
   c.out = o_part;
   c.lse = lse_part;
   c.status = status;
-  rc = ctx_attn_tc_supported(dtype, head_dim) ? launch_ctx_attn_tc(c, s) : launch_ctx_attn_simt(c, s);
+  rc = ctx_attn_tc_supported(dtype, head_dim) ? launch_ctx_attn_tc(c, s) : launch_ctx_attn_fma(c, s);
   if (rc) return rc;
 
   BufMergeArgs b;

@@ -1,4 +1,4 @@
-// Whole-sequence decode on fp32 FMA (fp32 mode, and bf16 mode for models outside the tensor-core chain).
+// Whole-sequence decode on fp32 FMA, in fp32 and in bf16 mode, for the jobs it is the faster path of (seq.cu).
 //
 // A launch-per-layer decode step spends its time on dependent launches and on a few CTAs walking all
 // the weights: at 64 streams of a 6-layer d_model 128 model a layer took 116 us for 20 us worth of
