@@ -133,6 +133,7 @@ struct SmemConfig {
     if (e == cudaSuccess && several_per_sm)
       e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
     if (e == cudaSuccess && tracked) bytes[dev] = smem;
+    if (e != cudaSuccess) cudaGetLastError();
     return e;
   }
 };
@@ -162,7 +163,9 @@ inline cudaError_t launch_dependent_cluster(void (*kernel)(P...), dim3 grid, dim
   }
   cfg.attrs = attr;
   cfg.numAttrs = n;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  if (e != cudaSuccess) cudaGetLastError();  // reported by the caller: it must not surface in someone else's next check
+  return e;
 }
 
 template <typename... P, typename... A>

@@ -68,3 +68,15 @@ def test_whole_sequence_path_after_a_smaller_job_of_the_queried_variant():
         _sample(eight)
         return int(lib.artab_sequence_workspace(eight._packed(eight._device).ref, C.byref(eight._state)))
     assert _on_a_thread(applies) > 0
+
+
+def test_a_refused_launch_does_not_surface_in_the_callers_next_operation():
+    """More heads than a grid has rows: the launch is refused on the host, nothing runs."""
+    from ar_tabpfn import _lib
+    lib = _lib.lib()
+    b = torch.zeros(64, dtype=torch.bfloat16, device="cuda")
+    f = torch.zeros(64, device="cuda")
+    with pytest.raises(_lib.ArtabError):
+        _lib.check(lib.artab_context_attention(_lib.BF16, _lib.ptr(b), _lib.ptr(b), _lib.ptr(b), 1, 1, 1, 70000, 32, 8, 8, 1,
+                                               _lib.ptr(f), _lib.ptr(f), None, _lib.stream_ptr()))
+    assert float((f + 1).sum()) == 64.0
