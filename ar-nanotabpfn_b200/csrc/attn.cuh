@@ -16,7 +16,7 @@ struct CtxAttnArgs {
   int out_lane_major; // n_splits == 1 only: write the [rows][H*Dh] result in the lane-major layout
   float* lse;         // [splits][rows][H]
   int32_t* status;    // device status word (bounded waits), may be null for SIMT
-  // Optional, tensor-core kernel: every CTA stores 0, or 1 when one of its waits gave up (its rows then have an LSE of
+  // Optional, tensor-core kernel on the caller's own K / V (not v_transposed): every CTA stores 0, or 1 when one of its waits gave up (its rows then have an LSE of
   // +inf, which makes their merged result NaN).  ctx_attn_tc_ctas words that need no clearing beforehand.
   int32_t* cta_status;
   int kv_stable;      // k_ctx / v_ctx were not written by the kernel launched just before this one

@@ -59,7 +59,7 @@ struct __align__(1024) Smem {
   float xmax[2][2][BM];             // row maxima exchanged between the two softmax warpgroups
   float xsum[BM];                   // row sum of the second warpgroup (epilogue)
   uint32_t tmem_base;
-  int redo;
+  int redo, look;
   WaitCtl ctl;
 };
 
@@ -447,7 +447,8 @@ ctx_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       for (int i = 0; i < DH / 4; ++i) o[i] = make_float4(0.f, 0.f, 0.f, 0.f);
       p.lse[out_row] = -INFINITY;
     }
-    if (threadIdx.x == 0 && p.cta_status) p.cta_status[(blockIdx.z * gridDim.y + h) * gridDim.x + blockIdx.x] = 0;
+    if constexpr (NATURAL)
+      if (threadIdx.x == 0 && p.cta_status) p.cta_status[(blockIdx.z * gridDim.y + h) * gridDim.x + blockIdx.x] = 0;
     return;
   }
 
@@ -459,6 +460,7 @@ ctx_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     mbar_init(&sm->s_free, 256);
     mbar_init(&sm->verdict, 256);
     sm->redo = 0;
+    sm->look = 0;
     for (int s = 0; s < NSTAGE; ++s) {
       mbar_init(&sm->kv_full[s], 1);
       mbar_init(&sm->kv_empty[s], 1);
@@ -587,39 +589,65 @@ ctx_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     float m = -INFINITY, l = 0.f;
     uint32_t r[32];
     bool ok = true;
-    // On an abort the loops still run every iteration (waits return at once, results are void):
+    // On an abort the loop still runs every iteration (waits return at once, results are void):
     // both warpgroups must execute the same number of bar.sync instructions.
-#pragma unroll 1
-    for (int i0 = 0;; i0 = nt) {   // first walk over the keys, second one
-#pragma unroll 1
-      for (int j = 0; j < nt; ++j) {
-        const int i = i0 + j;
-        ok = mbar_wait(&sm->s_full, i & 1, abort_flag) && ok;
-        tc_fence_after();
-        const int n_valid = p.n_ctx - (tile_begin + j) * BN;
-        if (j == 0 || i0) {
-          if (n_valid >= BN)
-            ok = softmax_tile<false, NATURAL>(sm, t_row, wg, row, i & 1, sc, BN, m, l, j == 0, abort_flag) && ok;
-          else
-            ok = softmax_tile<true, NATURAL>(sm, t_row, wg, row, i & 1, sc, n_valid, m, l, j == 0, abort_flag) && ok;
-        } else {
-          if (n_valid >= BN)
-            ok = softmax_tile_one_pass<false>(sm, t_row, wg, (i & 1) ^ 1, sc, BN, m, l, abort_flag) && ok;
-          else
-            ok = softmax_tile_one_pass<true>(sm, t_row, wg, (i & 1) ^ 1, sc, n_valid, m, l, abort_flag) && ok;
-        }
-        tmem_wait_st();
-        tc_fence_before();
-        mbar_arrive(&sm->p_full);
-      }
-      if (wg == 1) sm->xsum[row] = l;
-      const bool one_pass = nt > 1 && i0 == 0;
-      if (one_pass && !(l < kOnePassMax)) sm->redo = 1;
-      asm volatile("bar.sync 2, 256;" ::: "memory");
-      ok = mbar_wait(&sm->o_full, (i0 + nt - 1) & 1, abort_flag) && ok;  // the last P . V is done
+    int last = nt - 1;   // number of the last tile walked
+    for (int i = 0; i <= last; ++i) {
+      const int j = i < nt ? i : i - nt;
+      ok = mbar_wait(&sm->s_full, i & 1, abort_flag) && ok;
       tc_fence_after();
-      if (wg == 0) {
-        l += sm->xsum[row];
+      const int n_valid = p.n_ctx - (tile_begin + j) * BN;
+      if (j == 0 || i >= nt) {
+        if (n_valid >= BN)
+          ok = softmax_tile<false, NATURAL>(sm, t_row, wg, row, i & 1, sc, BN, m, l, j == 0, abort_flag) && ok;
+        else
+          ok = softmax_tile<true, NATURAL>(sm, t_row, wg, row, i & 1, sc, n_valid, m, l, j == 0, abort_flag) && ok;
+      } else {
+        if (n_valid >= BN)
+          ok = softmax_tile_one_pass<false>(sm, t_row, wg, (i & 1) ^ 1, sc, BN, m, l, abort_flag) && ok;
+        else
+          ok = softmax_tile_one_pass<true>(sm, t_row, wg, (i & 1) ^ 1, sc, n_valid, m, l, abort_flag) && ok;
+      }
+      tmem_wait_st();
+      tc_fence_before();
+      mbar_arrive(&sm->p_full);
+      if (i == nt - 1 && nt > 1) {
+        if (!(l <= 256.0f * 64 * nt)) {          // more than the two-pass form lets this half of the row grow to
+          sm->look = 1;
+          if (!(l < kOnePassMax)) sm->redo = 1;
+        }
+        asm volatile("bar.sync 2, 256;" ::: "memory");   // never times out: both warpgroups take the same decision
+        int redo = *(volatile int*)&sm->redo;
+        if (!redo && *(volatile int*)&sm->look) {   // rare: l is finite, l times a large V need not be
+          ok = mbar_wait(&sm->o_full, i & 1, abort_flag) && ok;
+          tc_fence_after();
+          if (wg == 0) {
+            tmem_ld32(t_row + kColO, r);
+            tmem_wait_ld();
+#pragma unroll
+            for (int d = 0; d < DH; ++d)
+              if (!(fabsf(__uint_as_float(r[d])) <= 3.0e38f)) sm->redo = 1;
+          }
+          asm volatile("bar.sync 2, 256;" ::: "memory");
+          redo = *(volatile int*)&sm->redo;
+        }
+        mbar_arrive(&sm->verdict);
+        if (redo) {
+          last = 2 * nt - 1;
+          m = -INFINITY;
+          l = 0.f;
+          ok = mbar_wait(&sm->o_full, i & 1, abort_flag) && ok;  // the last P . V has read P
+          tc_fence_after();
+        }
+      }
+    }
+    if (wg == 1) sm->xsum[row] = l;
+    asm volatile("bar.sync 2, 256;" ::: "memory");
+    if (wg == 0) {
+      l += sm->xsum[row];
+      if (ok) ok = mbar_wait(&sm->o_full, last & 1, abort_flag);
+      if (ok) {
+        tc_fence_after();
         float o[DH];
         tmem_ld32(t_row + kColO, r);          // P . V_hi
         tmem_wait_ld();
@@ -631,13 +659,7 @@ ctx_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 #pragma unroll
           for (int d = 0; d < DH; ++d) o[d] += __uint_as_float(r[d]);
         }
-        if (one_pass) {   // l is finite up to 2^100 per row, l times V need not be
-          bool over = false;
-#pragma unroll
-          for (int d = 0; d < DH; ++d) over = over || !(fabsf(o[d]) <= 3.0e38f);
-          if (over) sm->redo = 1;
-        }
-        if (ok && row_valid) {   // a second walk writes them again
+        if (row_valid) {
           const float inv = 1.0f / l;
 #pragma unroll
           for (int d = 0; d < DH; d += 4) {
@@ -648,13 +670,6 @@ ctx_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           p.lse[out_row] = (m + log2f(l)) * kLn2;
         }
       }
-      if (!one_pass) break;
-      asm volatile("bar.sync 2, 256;" ::: "memory");   // never times out: both warpgroups take the same decision
-      const int redo = *(volatile int*)&sm->redo;
-      mbar_arrive(&sm->verdict);
-      if (!redo) break;
-      m = -INFINITY;
-      l = 0.f;
     }
   }
 
@@ -674,7 +689,7 @@ ctx_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     landed(&sm->q_full, 0);
     for (int j = max(0, issued - NSTAGE); j < issued; ++j) landed(&sm->kv_full[j % NSTAGE], (j / NSTAGE) & 1);
   }
-  if (p.cta_status) {
+  if (NATURAL && p.cta_status) {   // the packed instance has no such callers
     if (threadIdx.x == 0) p.cta_status[(blockIdx.z * gridDim.y + h) * gridDim.x + blockIdx.x] = sm->ctl.abort_flag ? 1 : 0;
     if (sm->ctl.abort_flag && row_valid) p.lse[out_row] = INFINITY;
   }
