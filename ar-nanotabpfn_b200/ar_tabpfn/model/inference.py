@@ -416,10 +416,6 @@ class ARTabPFNPredictor:
         K = int(self.head.num_components)
         if expo.shape != (Nt, B, K) or normal.shape != (Nt, B):
             raise ValueError("variates must be (expo [Nt,B,K], normal [Nt,B])")
-        # zeros: a call whose bounded wait gives up leaves no values of an earlier one in them
-        samples = torch.zeros(B, Nt, device=device, dtype=torch.float32)
-        logdens = torch.zeros(B, Nt, device=device, dtype=torch.float32)
-        comp = torch.zeros(B, Nt, device=device, dtype=torch.int32)
         st = self._state
         stream = _lib.stream_ptr()
 
@@ -430,6 +426,12 @@ class ARTabPFNPredictor:
                 torch.cuda.current_stream(device).wait_event(drawn[t])
 
         ws = self._sequence_workspace(int(lib.artab_sequence_workspace(pm.ref, C.byref(st))))
+        # A call whose bounded wait gives up leaves zeros, not values of an earlier call in the same memory: the
+        # one-launch decode stores them itself.
+        results = torch.zeros if ws is None else torch.empty
+        samples = results(B, Nt, device=device, dtype=torch.float32)
+        logdens = results(B, Nt, device=device, dtype=torch.float32)
+        comp = results(B, Nt, device=device, dtype=torch.int32)
         if ws is not None:
             pm.prepare_sequence()
             # one launch per chunk of draws (one in all when they are given)

@@ -326,6 +326,22 @@ __device__ long long g_seq_tl[256][16 * kSeqMaxLayers + 8];
 #define SEQ_TL(id) do { } while (0)
 #endif
 
+// Void results are zeros, not what the memory held before.  Out of line and from the arguments alone: nothing of it is
+// live while the kernel works.
+__device__ __noinline__ void zero_results(const SeqArgs& a) {
+  uint32_t rank;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  const int stream0 = (int)(blockIdx.x / a.C) * a.spc, n = a.t1 - a.t0;
+  if (rank != 0) return;
+#pragma unroll 1
+  for (int i = threadIdx.x; i < min(a.spc, a.B - stream0) * n; i += kT + 32) {
+    const size_t o = (size_t)(stream0 + i / n) * a.Nt + a.t0 + i % n;
+    a.samples[o] = 0.f;
+    if (a.logdens) a.logdens[o] = 0.f;
+    if (a.comp) a.comp[o] = 0;
+  }
+}
+
 template <typename CT, int DH, int R, bool SHARED>
 __global__ void __launch_bounds__(kT + 32, 1) seq_simt_kernel(const __grid_constant__ SeqArgs a) {
   constexpr int S = R / 2;              // streams this variant holds (a.spc of them in use)
@@ -814,6 +830,7 @@ __global__ void __launch_bounds__(kT + 32, 1) seq_simt_kernel(const __grid_const
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (bars->abort_flag) {
     if (tid == 0 && a.status) atomicExch(a.status, 4);
+    zero_results(a);
     const long long t0 = clock64();
     while (clock64() - t0 < 100000) {
     }

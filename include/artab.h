@@ -218,6 +218,7 @@ ARTAB_API int64_t artab_sequence_workspace(const artab_model* m, const artab_sta
  *   expo [Nt][B][K], normal [Nt][B]: random numbers of ALL targets; the rest as in artab_decode_step.
  * A sequence may be decoded in several consecutive parts; the call with t0 = 0 lays the context out in
  * `workspace`, which must stay untouched until the last part.
+ * When a bounded wait gives up, the results of the streams it concerns are zero.
  * Replaces the loop of ARTabPFNPredictor.sample_sequence (ar_tabpfn/model/inference.py:323-366). */
 ARTAB_API int artab_decode_sequence(const artab_model* m, artab_state* st, const float* xt, int64_t xt_stride, int n_feat,
                           int n_targets, int t0, int t1, float* samples, const float* expo, const float* normal,
